@@ -148,6 +148,7 @@ struct Engine {
     int64_t ex_lo = 0, ex_hi = -1;  // and the .bim markers it left out (a chromosome, or none)
     float* dp = nullptr;          // mg: d' = 1/sd'^2 (0 off the subset's GRM markers)
     float* p2 = nullptr;          // mg: 2p'
+    double* p2d = nullptr;        // the same in FP64
     float* lut = nullptr;         // mg x 4: d' (g - 2p')^2 per packed code (diagonal)
     int32_t* flips = nullptr;     // fill-changed markers (room for every marker)
     float* dfill = nullptr;
@@ -184,6 +185,8 @@ struct Engine {
   double* spart = nullptr;        // column partials: cap_cols x max(blocks over np, over mg)
   float* smax = nullptr;          // FP16 / E4M3 form: column block maxima, as spart
   float* sscale = nullptr;        //   and the columns' power-of-two scales s1, s2 (2 x cap_cols)
+  bool digits = false;            // products on the FP4 pipe (the FP32 drop-ins, DigitsScope)
+  Fp4Scratch f4;
   float* sdiag_part[kSetupStreams] = {};  // per-chunk partial sums of a subset's diagonal, per set-up stream
 
 };
@@ -265,6 +268,9 @@ struct sg_ctx {
   void* d_G = nullptr;   // genotype matrix: BF16 (form 0) or FP16 then E4M3 (form 1), both layouts each
   int g_form = 0;
   int64_t mg = 0;
+  // the same values in E2M1 for the FP32 drop-ins' products (k_fp4.cu), built at the first of them
+  void* d_G4 = nullptr;
+  bool g4_refused = false;  // no memory for it: those products run as the others
   // synthetic bed image
   uint8_t* d_synth = nullptr;
   uint64_t synth_len = 0;
@@ -477,6 +483,7 @@ static int ensure_k_bf16(sg_ctx* c, bool want);
 static void engine_free(sg_ctx* c);
 
 static int ensure_g(sg_ctx* c, int form);
+static void free_g(sg_ctx* c);
 
 // the subset-exact engines (BF16 products, or FP16 high / E4M3 low)
 static bool exact_mode(int mode) { return mode == SG_MV_SUBSET_EXACT || mode == SG_MV_SUBSET_EXACT_F8; }
@@ -516,8 +523,7 @@ extern "C" int sg_set_matvec_mode(sg_ctx* c, int mode) {
   }
   if (was_exact) {  // the genotype matrix (2 bytes per sample and marker, twice) leaves HBM
     SG_TRY(sync(c));
-    dev_free(c, c->d_G);
-    c->d_G = nullptr;
+    free_g(c);
   }
   if (!c->have_grm) return SG_OK;
   SG_TRY(ensure_k_split(c, mode == SG_MV_TF32X3_TC));
@@ -530,8 +536,7 @@ static int ensure_g(sg_ctx* c, int form) {
   if (c->d_G && c->g_form == form) return SG_OK;
   if (c->d_G) {  // the other form's matrix leaves HBM first
     SG_TRY(sync(c));
-    dev_free(c, c->d_G);
-    c->d_G = nullptr;
+    free_g(c);
   }
   const int64_t np = round_up(c->nn, kRowTile), mg = round_up(std::max<int64_t>(c->m_bim, 1), kRowTile);
   if (c->have_grm && c->np != np) return set_err(c, SG_ERR_STATE, "GRM row padding differs");
@@ -556,6 +561,13 @@ static int ensure_g(sg_ctx* c, int form) {
   c->t_build[3] = ev_ms(c->tev[0], c->tev[1]);
   c->mg = mg;
   return SG_OK;
+}
+
+static void free_g(sg_ctx* c) {
+  dev_free(c, c->d_G);
+  dev_free(c, c->d_G4);
+  c->d_G = c->d_G4 = nullptr;
+  c->g4_refused = false;
 }
 
 extern "C" int sg_ctx_make_current(sg_ctx* c) {
@@ -657,8 +669,7 @@ static void free_geno(sg_ctx* c) {
   dev_free_t(c, c->d_codes);
   dev_free_t(c, c->d_vrflag_all);
   dev_free_t(c, c->d_fill_all);
-  dev_free(c, c->d_G);
-  c->d_G = nullptr;
+  free_g(c);
   c->fill_all.clear();
   c->have_geno = false;
   c->have_grm = false;
@@ -1151,6 +1162,65 @@ static cudaError_t d2h(sg_ctx* c, void* dst, const void* src, size_t bytes, cuda
   return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
 }
 
+static void fp4_free(sg_ctx* c) {
+  Fp4Scratch& w = c->eng.f4;
+  dev_free(c, w.Vq);
+  dev_free(c, w.Tq);
+  for (float** p : {&w.T, &w.U, &w.pmax, &w.mean, &w.descale1, &w.descale2}) dev_free_t(c, *p);
+  for (double** p : {&w.part, &w.qsum}) dev_free_t(c, *p);
+  w = Fp4Scratch{};
+}
+
+// The E2M1 genotype matrix and the scratch of the FP4 products; false when there is no memory (or
+// budget) for them, and the products then run as the engine's others do.
+static bool fp4_ready(sg_ctx* c) {
+  Engine& e = c->eng;
+  if (c->d_G4 && e.f4.T) return true;
+  if (c->g4_refused) return false;
+  const int64_t mm = fp4_matrix_bytes(c->mg, c->nn), cap = e.cap_cols + kFp4PadCols;
+  const int64_t nb = cap * fp4_nblk(e.np, c->mg);
+  Fp4Scratch& w = e.f4;
+  const bool build = !c->d_G4;
+  auto all = [&]() -> int {
+    if (build) SG_TRY(dev_alloc(c, &c->d_G4, (size_t)(mm + fp4_matrix_bytes(e.np, c->m_bim))));
+    SG_TRY(dev_alloc(c, &w.Vq, (size_t)fp4_digit_bytes(cap, c->nn)));
+    SG_TRY(dev_alloc(c, &w.Tq, (size_t)fp4_digit_bytes(cap, c->m_bim)));
+    SG_TRY(dev_alloc_t(c, &w.U, (size_t)(cap * e.np)));
+    SG_TRY(dev_alloc_t(c, &w.part, (size_t)nb));
+    SG_TRY(dev_alloc_t(c, &w.qsum, (size_t)nb));
+    SG_TRY(dev_alloc_t(c, &w.pmax, (size_t)nb));
+    for (float** p : {&w.mean, &w.descale1, &w.descale2}) SG_TRY(dev_alloc_t(c, p, (size_t)cap));
+    return dev_alloc_t(c, &w.T, (size_t)(cap * c->mg));
+  };
+  const std::string err = c->err;
+  if (all() != SG_OK) {
+    fp4_free(c);
+    if (build) {
+      dev_free(c, c->d_G4);
+      c->d_G4 = nullptr;
+    }
+    c->g4_refused = true;
+    c->err = err;
+    return false;
+  }
+  if (build) {
+    uint8_t* g = static_cast<uint8_t*>(c->d_G4);
+    launch_fp4_gbuild(c->d_codes, c->pitch, c->d_fill_all, c->m_bim, c->nn, g, g + mm, c->stream);
+    c->launches += 2;
+  }
+  return true;
+}
+
+// While it lives, the subset-exact engine's products run on the FP4 pipe (k_fp4.cu).  The drop-ins
+// that return FP32, as the reference's entry points do, hold one; the FP64 interfaces (the engine,
+// sg_pcg_solve, sg_grm_matmul and the batched fits over them) keep the BF16 products, and with them
+// their results bit for bit.
+struct DigitsScope {
+  Engine& e;
+  explicit DigitsScope(sg_ctx* c) : e(c->eng) { e.digits = c->mv_mode == SG_MV_SUBSET_EXACT; }
+  ~DigitsScope() { e.digits = false; }
+};
+
 static void engine_free(sg_ctx* c) {
   Engine& e = c->eng;
   cudaStreamSynchronize(c->side);
@@ -1174,7 +1244,7 @@ static void engine_free(sg_ctx* c) {
   dev_free_t(c, e.pcache);
   e.pcache_key.clear();
   for (auto& ss : e.sub) {
-    dev_free_t(c, ss.dp); dev_free_t(c, ss.p2); dev_free_t(c, ss.lut); dev_free_t(c, ss.flips);
+    dev_free_t(c, ss.dp); dev_free_t(c, ss.p2); dev_free_t(c, ss.p2d); dev_free_t(c, ss.lut); dev_free_t(c, ss.flips);
     dev_free_t(c, ss.dfill); dev_free_t(c, ss.bits); dev_free_t(c, ss.diag);
     dev_free_t(c, ss.qc); dev_free_t(c, ss.flag); dev_free_t(c, ss.mb); dev_free_t(c, ss.d_counts);
     if (ss.h_counts) cudaFreeHost(ss.h_counts);
@@ -1195,6 +1265,7 @@ static void engine_free(sg_ctx* c) {
   dev_free_t(c, e.smax);
   dev_free_t(c, e.sscale);
   for (auto& p : e.sdiag_part) dev_free_t(c, p);
+  fp4_free(c);
 
   e.dots_cap_sx = e.dots_cap_part = e.dots_cap_cols = 0;
   for (auto& dp : e.dots) {
@@ -1326,7 +1397,8 @@ static int engine_reserve(sg_ctx* c, int64_t max_columns, int64_t max_phenos) {
   if (!e.ev_up) SG_CUDA(c, cudaEventCreateWithFlags(&e.ev_up, cudaEventDisableTiming));
   e.have_prev = false;
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_pin), max_columns * sizeof(ColState), cudaHostAllocDefault));
-  SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_gcols), max_columns * sizeof(int32_t), cudaHostAllocDefault));
+  SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_gcols), (max_columns + kFp4PadCols) * sizeof(int32_t),
+                           cudaHostAllocDefault));
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_sst), max_columns * sizeof(ColState), cudaHostAllocDefault));
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_scol), max_columns * sizeof(int32_t), cudaHostAllocDefault));
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_acols), e.stage_cols * sizeof(int32_t), cudaHostAllocDefault));
@@ -1337,7 +1409,7 @@ static int engine_reserve(sg_ctx* c, int64_t max_columns, int64_t max_phenos) {
   SG_TRY(dev_alloc_t(c, &e.d_scol, (size_t)max_columns));
   for (auto& p : e.d_wstage) SG_TRY(dev_alloc_t(c, &p, (size_t)(2 * np)));
   SG_TRY(dev_alloc_t(c, &e.d_wstage2, (size_t)(2 * np)));
-  SG_TRY(dev_alloc_t(c, &e.d_gcols, (size_t)max_columns));
+  SG_TRY(dev_alloc_t(c, &e.d_gcols, (size_t)(max_columns + kFp4PadCols)));
   e.h_st.assign(max_columns, ColState{});
   for (auto& s : e.h_st) { s.kind = -1; s.active = 0; }
   SG_CUDA(c, cudaMemcpyAsync(e.d_st, e.h_st.data(), max_columns * sizeof(ColState), cudaMemcpyHostToDevice, c->stream));
@@ -1401,6 +1473,7 @@ static int subset_prepare(sg_ctx* c, int64_t slot, const uint8_t* mask) {
   if (!ss.ev_prep) SG_CUDA(c, cudaEventCreateWithFlags(&ss.ev_prep, cudaEventDisableTiming));
   if (!ss.dp) SG_TRY(dev_alloc_t(c, &ss.dp, (size_t)mg));
   if (!ss.p2) SG_TRY(dev_alloc_t(c, &ss.p2, (size_t)mg));
+  if (!ss.p2d) SG_TRY(dev_alloc_t(c, &ss.p2d, (size_t)mg));
   if (!ss.lut) SG_TRY(dev_alloc_t(c, &ss.lut, (size_t)(4 * mg)));
   if (!ss.diag) SG_TRY(dev_alloc_t(c, &ss.diag, (size_t)np));
   if (!ss.flips) SG_TRY(dev_alloc_t(c, &ss.flips, (size_t)std::max<int64_t>(m, 1)));
@@ -1417,7 +1490,7 @@ static int subset_prepare(sg_ctx* c, int64_t slot, const uint8_t* mask) {
                    c->qc_min_mac_vr, c->qc_max_mac_vr, c->qc_is_var_ratio, ss.qc, st);
   // d' = 1/sd'^2, 2p' and the diagonal table per marker, the fill-changed markers in marker order,
   // on the device (setGenoObj's per-marker values over the subset, FIT.cpp:436-495, 152-159)
-  launch_subset_derive(ss.qc, c->d_fill_all, m, mg, c->sub_loco_lo, c->sub_loco_hi, ss.dp, ss.p2, ss.lut, ss.flag,
+  launch_subset_derive(ss.qc, c->d_fill_all, m, mg, c->sub_loco_lo, c->sub_loco_hi, ns, ss.dp, ss.p2, ss.p2d, ss.lut, ss.flag,
                        ss.flips, ss.dfill, ss.d_counts, st);
   SG_CUDA(c, cudaMemcpyAsync(ss.h_counts, ss.d_counts, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   SG_CUDA(c, cudaEventRecord(ss.ev_prep, st));
@@ -1480,6 +1553,7 @@ static int subset_setup(sg_ctx* c, int64_t slot, const uint8_t* mask, const uint
   SG_LAUNCHED(c, W > 0 ? 1 : 0);
   ss.dev.dprime = ss.dp;
   ss.dev.p2 = ss.p2;
+  ss.dev.p2d = ss.p2d;
   ss.dev.flips = ss.flips;
   ss.dev.dfill = ss.dfill;
   ss.dev.bits = ss.bits;
@@ -2040,6 +2114,20 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
       return SG_OK;
     }
     const int64_t np = e.np, mg = c->mg;
+    if (e.digits && fp4_ready(c)) {
+      const int ct = fp4_tile_cols(nact);
+      const int64_t npad = round_up(nact, ct);
+      for (int64_t j = nact; j < npad; ++j) e.h_gcols[j] = -1;
+      SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, npad * 4, cudaMemcpyHostToDevice, c->stream));
+      int nl = 0;
+      const uint8_t* g4 = static_cast<const uint8_t*>(c->d_G4);
+      const cudaError_t err = fp4_product(g4, g4 + fp4_matrix_bytes(mg, c->nn), e.Pf, np, c->nn, mg, c->m_bim, e.d_gcols,
+                                          npad, ct, e.d_st, e.d_slots, e.winv, e.max_w, e.f4, e.Yf, c->stream, &nl);
+      if (err != cudaSuccess) return set_err(c, SG_ERR_CUDA, "tcgen05 genotype GEMM: %s", cudaGetErrorString(err));
+      SG_LAUNCHED(c, nl);
+      *launched = npad;
+      return SG_OK;
+    }
     const int64_t npad = tc_grmv_padded_cols(round_up(nact, 32), e.cap_cols, np, kTilesSplitB, c->num_sms);
     for (int64_t j = nact; j < npad; ++j) e.h_gcols[j] = -1;
     SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, npad * 4, cudaMemcpyHostToDevice, c->stream));
@@ -2999,6 +3087,7 @@ extern "C" int sg_grm_matmul(sg_ctx* c, const double* V, int64_t k, double* out)
 
 extern "C" int sg_getCrossprodMatAndKin(sg_ctx* c, const float* b, float* out) {
   NEED_OPERATOR(c);
+  DigitsScope digits(c);
   std::vector<double> bd, od(c->nn);
   f2d(b, c->nn, bd);
   SG_TRY(sg_grm_matmul(c, bd.data(), 1, od.data()));
@@ -3049,6 +3138,7 @@ extern "C" int sg_pcg_solve(sg_ctx* c, const double* w, const double* tau, const
 static int solve_f32(sg_ctx* c, const float* w, const float* tau, const float* B, int64_t k, int maxiter,
                      float tol, float* out, int32_t* iters) {
   NEED_OPERATOR(c);
+  DigitsScope digits(c);
   const int64_t n = c->nn;
   if (!all_finite(w, n) || !all_finite(tau, 2)) return set_err(c, SG_ERR_NUMERIC, "W or tau not finite");
   std::vector<double> wd, bd, xd(n * k);
@@ -3114,6 +3204,7 @@ static int trace_common(sg_ctx* c, const float* Sigma_iX, int64_t p, const float
                         bool quant, float* trace, int32_t* nrun_used) {
   NEED_OPERATOR(c);
   if (nrun < 2) return set_err(c, SG_ERR_INVALID, "nrun must be >= 2");
+  DigitsScope digits(c);
   SG_TRY(dropin_setup(c, w, tau, 2 * nrun + 4));
   std::vector<double> SX, cv;
   f2d(Sigma_iX, c->nn * p, SX);
@@ -3156,6 +3247,7 @@ int ai_score(sg_ctx* c, const float* Y, const float* X, int64_t p, const float* 
              const float* Sigma_iY, const float* Sigma_iX, const float* cov_in, int nrun, int maxiter,
              float tol, float cutoff, uint64_t seed, bool quant, AIOut* o) {
   NEED_OPERATOR(c);
+  DigitsScope digits(c);
   const int64_t n = c->nn;
   SG_TRY(dropin_setup(c, w, tau, 2 * nrun + 8));
   std::vector<double> Yd, Xd, SY, SX, cv;

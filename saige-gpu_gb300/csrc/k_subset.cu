@@ -129,18 +129,20 @@ void launch_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int
 
 // A subset's GRM tables from its per-marker QC records, as setgeno over the subset builds them
 // (the LUT's 2p and 1/sd: FIT.cpp:152-159): for each GRM marker of the subset, d' = (1/sd')^2,
-// 2p', and lut4 = d' (g - 2p')^2 for the four packed codes (00 -> 2, 01 -> the subset's own fill,
+// 2p' (in FP32 as the reference's LUT, and in FP64 from the allele count: the mean genotype), and lut4 = d' (g - 2p')^2 for the four packed codes (00 -> 2, 01 -> the subset's own fill,
 // 10 -> 1, 11 -> 0); zeros elsewhere and past m.  flag bit 0: a GRM marker whose subset fill
 // differs from the cohort fill G holds; bit 1: a GRM marker of the subset.  Markers ex_lo..ex_hi
 // (one chromosome left out; none when ex_lo > ex_hi) are not GRM markers of the subset: the
 // subset's GRM over the remaining markers is K_-j of setStartEndIndex + parallelCrossProd_LOCO
 // (FIT.cpp:3067-3085, 1790-1851), its diagonal that of set_Diagof_StdGeno_LOCO (FIT.cpp:4934-4959).
 __global__ void subset_derive_kernel(const MarkerQC* __restrict__ qc, const int32_t* __restrict__ fill_all,
-                                     int64_t m, int64_t mg, int64_t ex_lo, int64_t ex_hi, float* __restrict__ dp,
-                                     float* __restrict__ p2, float4* __restrict__ lut4, uint8_t* __restrict__ flag) {
+                                     int64_t m, int64_t mg, int64_t ex_lo, int64_t ex_hi, double ns,
+                                     float* __restrict__ dp, float* __restrict__ p2, double* __restrict__ p2d,
+                                     float4* __restrict__ lut4, uint8_t* __restrict__ flag) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= mg) return;
   float d32 = 0.0f, tp = 0.0f;
+  double tpd = 0.0;
   float4 l = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   uint8_t f = 0;
   if (k < m && (k < ex_lo || k > ex_hi)) {
@@ -150,6 +152,7 @@ __global__ void subset_derive_kernel(const MarkerQC* __restrict__ qc, const int3
       const float two_p = 2.0f * q.freq;
       d32 = (float)d;
       tp = two_p;
+      tpd = (double)q.allele / ns;
       const double t0 = 2.0 - (double)two_p, t1 = (double)q.fill - (double)two_p;
       const double t2 = 1.0 - (double)two_p, t3 = 0.0 - (double)two_p;
       l.x = (float)(d * t0 * t0);
@@ -161,6 +164,7 @@ __global__ void subset_derive_kernel(const MarkerQC* __restrict__ qc, const int3
   }
   dp[k] = d32;
   p2[k] = tp;
+  p2d[k] = tpd;
   lut4[k] = l;
   flag[k] = f;
 }
@@ -214,10 +218,10 @@ subset_flips_kernel(const MarkerQC* __restrict__ qc, const int32_t* __restrict__
 }
 
 void launch_subset_derive(const MarkerQC* qc, const int32_t* fill_all, int64_t m, int64_t mg, int64_t ex_lo,
-                          int64_t ex_hi, float* dp, float* p2, float* lut4, uint8_t* flag, int32_t* flips, float* dfill,
-                          int64_t* counts, cudaStream_t s) {
+                          int64_t ex_hi, int64_t ns, float* dp, float* p2, double* p2d, float* lut4, uint8_t* flag,
+                          int32_t* flips, float* dfill, int64_t* counts, cudaStream_t s) {
   subset_derive_kernel<<<(unsigned)((mg + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-      qc, fill_all, m, mg, ex_lo, ex_hi, dp, p2, reinterpret_cast<float4*>(lut4), flag);
+      qc, fill_all, m, mg, ex_lo, ex_hi, (double)ns, dp, p2, p2d, reinterpret_cast<float4*>(lut4), flag);
   subset_flips_kernel<<<1, kFlipThreads, 0, s>>>(qc, fill_all, flag, m, flips, dfill, counts);
 }
 

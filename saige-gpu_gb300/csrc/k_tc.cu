@@ -41,6 +41,7 @@
 //     RHS-major so each TMEM column is a coalesced row of Y^T; split variants
 //     with TF32 or BF16 high/low halves of K and P (three products).
 #include "sg_internal.h"
+#include "tc_common.cuh"
 #include <algorithm>
 
 #include <cuda.h>
@@ -55,6 +56,8 @@ namespace sg {
 
 namespace {
 
+using namespace tc;
+
 constexpr int kTileM = 128;
 // products per K step of the GEMM kernel (see tc_gemm_kernel)
 constexpr int kOne = 0, kSplitB = 1, kSplit3 = 2, kSplit4 = 3, kSplitB8 = 4;
@@ -65,7 +68,6 @@ __host__ __device__ constexpr bool form_has_b2(int f) { return f != kOne; }
 __host__ __device__ constexpr int form_rb2(int f, int rb) { return f == kSplitB8 ? rb / 2 : rb; }
 constexpr int kRowBytes = 128;                 // one SWIZZLE_128B atom row
 constexpr int kATileBytes = kTileM * kRowBytes;  // 16 KB
-constexpr unsigned long long kWaitBudgetNs = 4000000000ull;  // 4 s per wait
 // warp roles of the GEMM kernel: 8 drain/epilogue warps, the TMA producer, the MMA issuer
 constexpr int kDrainWarps = 8;
 constexpr int kProducerWarp = 8;
@@ -73,94 +75,6 @@ constexpr int kMmaWarp = 9;
 constexpr int kGemmThreads = 320;
 
 __device__ int g_tc_error = 0;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ unsigned long long gtimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait: returns false (and records ``code``) when the budget runs out
-// or another thread of this kernel already gave up.
-__device__ __forceinline__ bool mbar_wait_budget(uint64_t* bar, uint32_t parity, int code,
-                                                 volatile int* abort_flag, unsigned long long budget_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = gtimer();
-  for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 255u) == 0u) {
-      if (*abort_flag) return false;
-      if (gtimer() - t0 > budget_ns) {
-        *abort_flag = 1;
-        atomicCAS(&g_tc_error, 0, code);
-        return false;
-      }
-    }
-  }
-}
-
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int code,
-                                          volatile int* abort_flag) {
-  return mbar_wait_budget(bar, parity, code, abort_flag, kWaitBudgetNs);
-}
-
-// Bounded wait with a sleeping back-off between polls, for waits that last a whole chunk of MMAs:
-// the drain warps share the SM's schedulers with the single-lane TMA and MMA loops.
-__device__ __forceinline__ bool mbar_wait_sleep(uint64_t* bar, uint32_t parity, int code,
-                                                volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = gtimer();
-  unsigned ns = 32;
-  for (;;) {
-    __nanosleep(ns);
-    if (mbar_try_wait(bar, parity)) return true;
-    if (ns < 256) ns <<= 1;
-    if (*abort_flag) return false;
-    if (gtimer() - t0 > kWaitBudgetNs) {
-      *abort_flag = 1;
-      atomicCAS(&g_tc_error, 0, code);
-      return false;
-    }
-  }
-}
-
-// Bounded wait at teardown: the MMAs a CTA issued complete within microseconds once issued (their
-// operands are already in shared memory), so this wait ignores the abort flag and gives up after
-// 1 s without recording anything.
-__device__ __forceinline__ void mbar_wait_teardown(uint64_t* bar, uint32_t parity) {
-  const unsigned long long t0 = gtimer();
-  while (!mbar_try_wait(bar, parity))
-    if (gtimer() - t0 > 1000000000ull) return;
-}
 
 // Self-test of the bounded wait: waits on an mbarrier that nothing arrives at, with a short budget,
 // and reports through the same error flag the GEMM kernels use.
@@ -173,15 +87,7 @@ __global__ void wait_selftest_kernel(unsigned long long budget_ns, int* waited_o
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  if (threadIdx.x == 0) *waited_out = mbar_wait_budget(&bar, 0u, 9, &abort_flag, budget_ns) ? 0 : 1;
-}
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar,
-                                            int32_t x, int32_t y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
+  if (threadIdx.x == 0) *waited_out = mbar_wait_budget(&bar, 0u, 9, &abort_flag, budget_ns, &g_tc_error) ? 0 : 1;
 }
 
 // Shared-memory matrix descriptor, K-major operand in SWIZZLE_128B layout:
@@ -263,63 +169,6 @@ __device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t a, uint64_t b,
         "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
   }
-}
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Address of the same shared-memory location in CTA ``rank`` of the cluster.
-__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-  return r;
-}
-
-// Arrive once on an mbarrier given by its cluster address (this CTA's or the peer's).
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
-}
-
-// CTA-pair load: the box lands in this CTA's shared memory and completes its transaction bytes on
-// the mbarrier at cluster address ``bar_cluster``, which may sit in the pair's other CTA.
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster,
-                                                 int32_t x, int32_t y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster), "r"(x), "r"(y)
-      : "memory");
-}
-
-template <bool kPair>
-__device__ __forceinline__ void umma_commit(uint32_t bar_cluster) {
-  if constexpr (kPair)
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 ::"r"(bar_cluster) : "memory");
-  else
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 ::"r"(bar_cluster) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 struct TileCoord {
@@ -443,7 +292,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       for (int kb = 0; kb < num_kb; ++kb) {
         const int s = kb % S;
         const uint32_t ph = (uint32_t)(kb / S) & 1u;
-        if (!mbar_wait(&empty[s], ph ^ 1u, 1, abort_flag)) break;
+        if (!mbar_wait(&empty[s], ph ^ 1u, 1, abort_flag, &g_tc_error)) break;
         uint8_t* st = smem + s * kStageBytes;
         const int32_t x = kb * (RB / (kTF32 ? 4 : 2));
         // box u of an operand covers K bytes [u kSW, (u + 1) kSW) of the stage's slice and sits
@@ -507,12 +356,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const int kin = kb - ch * drain_kb;
         const int ab = ch & 1;
         if (kin == 0) {
-          if (!mbar_wait(&acc_empty[ab], ((uint32_t)(ch >> 1) & 1u) ^ 1u, 5, abort_flag)) break;
+          if (!mbar_wait(&acc_empty[ab], ((uint32_t)(ch >> 1) & 1u) ^ 1u, 5, abort_flag, &g_tc_error)) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
         const int s = kb % S;
         const uint32_t ph = (uint32_t)(kb / S) & 1u;
-        if (!mbar_wait(&full[s], ph, 2, abort_flag)) break;
+        if (!mbar_wait(&full[s], ph, 2, abort_flag, &g_tc_error)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t dacc = tmem_base + (uint32_t)ab * kAccCols;
         const uint32_t a0 = smem_u32(smem + s * kStageBytes);
@@ -573,7 +422,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     for (int ch = 0; ch < nchunks; ++ch) {
       const int ab = ch & 1;
       // one lane polls; the others wait in the shuffle (warp-uniform: tcgen05.ld is .sync.aligned)
-      if (lane == 0) go = mbar_wait_sleep(&acc_full[ab], (uint32_t)(ch >> 1) & 1u, 3, abort_flag) && !*abort_flag;
+      if (lane == 0) go = mbar_wait_sleep(&acc_full[ab], (uint32_t)(ch >> 1) & 1u, 3, abort_flag, &g_tc_error) && !*abort_flag;
       go = __shfl_sync(0xffffffffu, go, 0);
       __syncwarp();
       if (!go) break;
@@ -1521,6 +1370,13 @@ cudaError_t tc_gemm_splitb8(const void* A, const void* A8, int64_t rows, int64_t
 }
 
 cudaError_t tc_check_error(cudaStream_t s) { return check_error_flag(s); }
+
+PFN_cuTensorMapEncodeTiled_v12000 tc::tc_encode_fn() { return encode_fn(); }
+
+int* tc::tc_error_flag() {
+  void* p = nullptr;
+  return cudaGetSymbolAddress(&p, g_tc_error) == cudaSuccess ? static_cast<int*>(p) : nullptr;
+}
 
 // ---------------------------------------------------------------- GRM.V that allocates nothing
 //

@@ -202,6 +202,7 @@ int64_t pcg_nblk(int64_t np);
 struct SubsetSlot {
   const float* dprime;    // mg: 1/sd'^2 of the subset's GRM markers, 0 for the others
   const float* p2;        // mg: 2 p' (the subset's allele frequency, FP32 as the reference's LUT)
+  const double* p2d;      // mg: 2 p' in FP64 (allele count / subset size)
   const int32_t* flips;   // nflip markers whose subset fill differs from the cohort fill in G
   const float* dfill;     // nflip: subset fill - cohort fill
   const uint32_t* bits;   // W x np (word-major): bit b of word w of sample i = i misses marker
@@ -217,8 +218,8 @@ void launch_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int
 // flag: mg bytes of scratch, flips / dfill: room for m entries, counts: 2 int64 on the device;
 // markers ex_lo..ex_hi are left out of the subset's GRM (none when ex_lo > ex_hi)
 void launch_subset_derive(const MarkerQC* qc, const int32_t* fill_all, int64_t m, int64_t mg, int64_t ex_lo,
-                          int64_t ex_hi, float* dp, float* p2, float* lut4, uint8_t* flag, int32_t* flips, float* dfill,
-                          int64_t* counts, cudaStream_t s);
+                          int64_t ex_hi, int64_t ns, float* dp, float* p2, double* p2d, float* lut4, uint8_t* flag,
+                          int32_t* flips, float* dfill, int64_t* counts, cudaStream_t s);
 void launch_subset_bitmap(const uint8_t* codes, int64_t pitch, const int32_t* flips, int nflip, int W,
                           const uint8_t* mask, int64_t nn, int64_t np, uint32_t* bits, cudaStream_t s);
 // part: subset_diag_scratch(m, np) floats of scratch
@@ -251,6 +252,33 @@ void launch_subset_finalize_f8(const float* U, int64_t np, int64_t nn, const int
                                const ColState* st, const SubsetSlot* slots, const void* Th, const void* Tl,
                                int64_t mg, const float* scale2, const double* part, const double* winv, float* Yf,
                                cudaStream_t s);
+
+// ---- exact-integer genotype GEMMs on the FP4 tensor pipe (k_fp4.cu)
+constexpr int kFp4StageK = 192;   // elements of K per pipeline stage
+constexpr int kFp4PadCols = 64;   // columns a launch may pad its last tile with
+int64_t fp4_matrix_bytes(int64_t rows, int64_t k);  // G in E2M1 stages: rows padded to 256, K to 192
+int64_t fp4_digit_bytes(int64_t cols, int64_t k);   // room for cols columns' digits, whatever the tile
+// G with rows of markers (m x nn) and with rows of samples (nn x m), missing calls at the cohort fill
+void launch_fp4_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int64_t m, int64_t nn, void* Gmm,
+                       void* Gsm, cudaStream_t s);
+// columns per tile for a launch over ncols columns (pad ncols to a multiple of it)
+int fp4_tile_cols(int64_t ncols);
+// Scratch of one subset-exact product over up to ``cap`` columns (cap counts the padding columns)
+struct Fp4Scratch {
+  void *Vq = nullptr, *Tq = nullptr;       // digits of the centred P and of T'
+  float *T = nullptr, *U = nullptr;        // cap x mg, cap x np
+  double *part = nullptr, *qsum = nullptr; // cap x nblk block partials each
+  float* pmax = nullptr;                   // the same size
+  float *mean = nullptr, *descale1 = nullptr, *descale2 = nullptr;  // cap each
+};
+// Y[cols[j]] = K_S P[cols[j]] on each column's subset; ncols a multiple of ct, padding columns have
+// cols[j] = -1.  Launches only (*launches of them): the caller reads the wait-error flag
+// (tc_check_error) once the stream has drained.
+int fp4_nblk(int64_t np, int64_t mg);  // block partials per column that the scratch holds
+cudaError_t fp4_product(const void* Gmm, const void* Gsm, const float* Pf, int64_t np, int64_t nn, int64_t mg,
+                        int64_t m, const int32_t* cols, int64_t ncols, int ct, const ColState* st,
+                        const SubsetSlot* slots, const double* winv, int max_w, const Fp4Scratch& w, float* Yf,
+                        cudaStream_t s, int* launches);
 constexpr int kProbeDotsMaxP = 16;
 // Per probe j (vecs[j] = Sigma^-1 u_j and vecs[k+j] = K u_j, u masked by minv != 0):
 // block partials of [Au.Su, u.Su, Au.SX_q (q < p), SX_q.u (q < p)] -> part[(j*nblk + b)*(2+2p) + v]

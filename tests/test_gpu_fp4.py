@@ -1,0 +1,103 @@
+"""Exact-integer genotype GEMMs (csrc/k_fp4.cu) through the subset-exact engine's FP32 drop-ins, at the
+edges of its row blocks (256), K stages (192), column tiles (16, 32, 48, 64) and of the exact range of
+one accumulation (2^20 elements)."""
+import numpy as np
+import pytest
+
+from oracle import aireml, plink
+from saigegpu import MV_FP32_SIMT, MV_SUBSET_EXACT, synth
+
+pytestmark = pytest.mark.gpu
+
+# A product's entries carry a bounded number of FP32 roundings (the column's fixed-point quantisation
+# at 2^-25 of its largest entry, T, d' T, 2p', U, the difference U - c and its scale): fewer than 64
+# of 2^-24, relative to the largest entry
+TOL = 64 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("n,m", [(33, 40), (128, 191), (129, 193), (256, 384), (385, 577), (1000, 2100)])
+def test_products_match_fp64_at_tile_edges(gpu_ctx, n, m):
+    """K b of one column, and two PCG iterations over 1 to 130 columns (a fixed count: the columns'
+    products enter with coefficients of order one, so twice two products' bound holds)."""
+    bed, _ = synth.synth_bed(500 + n, n, m, 0.03)
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    g = plink.setgeno(bed, n, m, np.arange(1, n + 1), np.ones(n, bool), 0.01, 0.15)
+    grm = aireml.DenseGRM(g)
+    rng = np.random.default_rng(n)
+    V = (rng.standard_normal((n, 130)) + 0.3).astype(np.float32)
+    V[:, 3] = 0.0
+    V[n // 2, 5] = 3000.0      # one entry far above the rest
+    V[:, 7] *= np.float32(1e-12)
+    V[:, 9] *= np.float32(1e12)
+    w, tau = np.ones(n, np.float32), np.array([0.5, 0.5], np.float32)
+    ref = aireml.pcg(grm, w, tau, V, 2, 0.0)
+    ctx.set_matvec_mode(MV_SUBSET_EXACT)
+    try:
+        for j in (0, 5, 9):
+            y, want = ctx.getCrossprodMatAndKin(V[:, j]), grm.K @ V[:, j].astype(np.float64)
+            assert np.abs(y - want).max() < TOL * np.abs(want).max(), j
+        first = None
+        for k in (1, 15, 16, 17, 32, 33, 48, 49, 64, 65, 130):
+            X = ctx.getSigma_X(w, tau, V[:, :k], 2, 0.0)
+            err = np.abs(X - ref[:, :k]).max(0) / (np.abs(ref[:, :k]).max(0) + 1e-300)
+            assert err.max() < 4 * TOL, (k, err.argmax(), err.max())
+            first = X[:, 0] if first is None else first
+            np.testing.assert_array_equal(X[:, 0], first)  # whatever the tile
+            if k > 3:
+                assert not X[:, 3].any()
+    finally:
+        ctx.set_matvec_mode(MV_FP32_SIMT)
+
+
+def test_reduction_longer_than_one_exact_accumulation(gpu_ctx):
+    """1,050,000 markers: the second product's K is accumulated in two segments."""
+    n, m = 192, 1_050_000
+    rng = np.random.default_rng(3)
+    p = rng.uniform(0.05, 0.5, (m, 1))
+    u = rng.random((m, n), dtype=np.float32)
+    g = (u >= (1 - p) ** 2).astype(np.uint8) + (u >= 1 - p * p).astype(np.uint8)
+    field = np.array([3, 2, 0], np.uint8)[g].reshape(m, n // 4, 4)
+    body = field[..., 0] | (field[..., 1] << 2) | (field[..., 2] << 4) | (field[..., 3] << 6)
+    bed = np.concatenate([np.array([0x6C, 0x1B, 0x01], np.uint8), body.ravel()])
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    V = rng.standard_normal((n, 3)).astype(np.float32)
+    ref, used = np.zeros((n, 3)), 0
+    for i in range(0, m, 50_000):
+        x = g[i:i + 50_000].astype(np.float64)
+        f = x.mean(1, keepdims=True) / 2
+        ok = (np.minimum(f, 1 - f) >= 0.01)[:, 0]
+        z = (x - 2 * f) / np.sqrt(2 * f * (1 - f))
+        ref += z[ok].T @ (z[ok] @ V)
+        used += int(ok.sum())
+    ref /= used
+    assert used == ctx.dims()["m_qc"]
+    ctx.set_matvec_mode(MV_SUBSET_EXACT)
+    try:
+        Y = np.column_stack([ctx.getCrossprodMatAndKin(V[:, j]) for j in range(3)])
+    finally:
+        ctx.set_matvec_mode(MV_FP32_SIMT)
+    assert (np.abs(Y - ref).max(0) / np.abs(ref).max(0)).max() < TOL
+
+
+def test_refused_memory_falls_back(gpu_ctx):
+    """A budget without room for the E2M1 matrix: the drop-ins run on the BF16 products instead."""
+    from saigegpu import Context
+    n, m = 500, 900
+    bed, _ = synth.synth_bed(9, n, m, 0.02)
+    b = np.random.default_rng(1).standard_normal(n).astype(np.float32)
+    out = []
+    for budget in (0, None):
+        with Context(0, 0 if budget == 0 else tight) as ctx:
+            ctx.setgeno(bed, n, m)
+            ctx.set_matvec_mode(MV_SUBSET_EXACT)
+            ctx.engine_reserve(128, 1)
+            ctx.grm_matmul(b)  # the BF16 products' scratch
+            tight = ctx.bytes_in_use() + (1 << 16)
+            out.append(ctx.getCrossprodMatAndKin(b))
+            if budget is None:
+                np.testing.assert_array_equal(out[1], ctx.grm_matmul(b).astype(np.float32))
+    np.testing.assert_allclose(out[0], out[1], rtol=0, atol=6e-5 * np.abs(out[0]).max())
