@@ -42,9 +42,12 @@ enum sg_status {
 
 /* GRM build precisions (sg_grm_build) */
 enum sg_grm_precision {
-  SG_GRM_FP32_SIMT = 0, /* FP32 standardised genotypes, FP32 CUDA-core SYRK */
+  SG_GRM_FP32_SIMT = 0, /* near-exact FP32 K: exact integer sums on the FP4 tensor pipe, rounded once, while
+                           the GRM markers' 1/sd^2 span at most a factor of 200; else FP32 standardised
+                           genotypes, FP32 CUDA-core SYRK */
   SG_GRM_BF16_TC = 1,   /* BF16 genotypes, tcgen05 SYRK, FP32 accumulation in TMEM */
-  SG_GRM_BF16X3_TC = 2  /* split-BF16 (hi+lo, 4 products) tcgen05 SYRK: 16-bit genotypes, near-FP64 K */
+  SG_GRM_BF16X3_TC = 2  /* as SG_GRM_FP32_SIMT, with a split-BF16 (hi+lo, 4 products) tcgen05 SYRK over
+                           16-bit genotypes in the place of the CUDA-core one */
 };
 
 /* GRM.V product engines used inside the PCG (sg_set_matvec_mode) */

@@ -35,8 +35,7 @@
 #include "sg_internal.h"
 #include "tc_common.cuh"
 
-#include <cudaTypedefs.h>
-#include <mutex>
+#include <cmath>
 
 namespace sg {
 
@@ -65,11 +64,11 @@ constexpr uint32_t kDigitBias = 62748517u;  // 13^7: makes q non-negative withou
 constexpr uint32_t kDiv13 = 330382100u;     // ceil(2^32 / 13): exact quotients below 2^30
 
 // seven E2M1 digit codes of q, lowest digit first, in the low 28 bits
-__device__ __forceinline__ uint32_t digit_codes(int32_t q) {
+__host__ __device__ __forceinline__ uint32_t digit_codes(int32_t q) {
   uint32_t x = (uint32_t)q + kDigitBias, w = 0;
 #pragma unroll
   for (int d = 0; d < kDigits; ++d) {
-    const uint32_t t = __umulhi(x, kDiv13);
+    const uint32_t t = (uint32_t)(((uint64_t)x * kDiv13) >> 32);
     const uint32_t r = x - 13u * t;
     w |= ((uint32_t)(kDigitCodes >> (4u * r)) & 15u) << (4 * d);
     x = t + ((kDigitCarry >> r) & 1u);
@@ -148,15 +147,43 @@ __device__ __forceinline__ void tmem_ld56(uint32_t taddr, uint32_t (&r)[56]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// What a tile's sums become: D = FP32 of sum x descale (kProduct); the 64-bit sums themselves (kSums); the
+// GRM's entries (kSyrk, see fp4_syrk).
+enum { kProduct = 0, kSums = 1, kSyrk = 2 };
+
+// kSyrk: tiles come from a table (row block, column tile), and entry (r, c), c <= r < n, is
+// (sum - shift[r] - shift[c] + c0) scale, written to K[r][c] and K[c][r] (rows past n: zero).
+struct SyrkArgs {
+  const int2* tiles;
+  const long long* shift;
+  long long c0;
+  float scale;
+  int64_t n;
+};
+
+// The sum of seven digits' accumulators: integers below 2^24 in units of 1/2.  ``magic``: below 2^22,
+// where adding 1.5 2^23 leaves the integer in the low mantissa bits (a conversion takes a quarter-rate
+// instruction).
+__device__ __forceinline__ long long combine_digits(const uint32_t* v, bool magic) {
+  long long t = 0;
+#pragma unroll
+  for (int d = kDigits - 1; d >= 0; --d) {
+    const float x = __uint_as_float(v[d]);
+    const int s = magic ? (__float_as_int(fmaf(x, 2.0f, 12582912.0f)) - 0x4B400000) : __float2int_rn(2.0f * x);
+    t = 13 * t + s;
+  }
+  return t;
+}
+
 // One 256-row x CT-column tile per CTA pair.  Warp 8 (one lane) loads a stage's rows of G and of the
 // digits into an S-stage ring (the pair's loads complete on the leader's barrier); warp 9 of the
 // leader issues two K = 96 MMAs per stage and 32-column half; warps 0-7 combine and store.
 // Tiles run column tiles fastest, so the pairs resident at one time share their strips of G in L2.
-template <int CT, int S>
+template <int CT, int S, int kMode>
 __global__ void __launch_bounds__(kFp4Threads, CT <= 32 ? 2 : 1)
 fp4_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int stages,
-                int ncolt, float* __restrict__ D, int64_t ldd, int64_t nrows, const float* __restrict__ descale,
-                int* __restrict__ err) {
+                int ncolt, void* __restrict__ Dv, int64_t ldd, int64_t nrows, const float* __restrict__ descale,
+                const SyrkArgs sy, int* __restrict__ err) {
   constexpr int kHalves = CT > 32 ? 2 : 1;
   constexpr int kN0 = CT >= 32 ? 224 : 112, kN1 = CT == 64 ? 224 : 112;
   constexpr int kBStage = 336 * CT;               // this CTA's digit rows (3.5 CT) per stage
@@ -177,7 +204,15 @@ fp4_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
   const uint32_t crank = cluster_rank();
   const bool leader = crank == 0;
   const int tile = blockIdx.x >> 1;
-  const int rt = tile / ncolt, bt = tile - rt * ncolt;
+  int rt, bt;
+  if constexpr (kMode == kSyrk) {
+    const int2 tc = sy.tiles[tile];
+    rt = tc.x;
+    bt = tc.y;
+  } else {
+    rt = tile / ncolt;
+    bt = tile - rt * ncolt;
+  }
   const int row_block = 2 * rt + (int)crank;
 
   if (threadIdx.x == 0) {
@@ -280,6 +315,7 @@ fp4_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const int64_t r = (int64_t)row_block * 128 + quad * 32 + lane;
     const uint32_t acce_leader = cluster_addr(acc_empty, 0);
     const int nseg = (stages + kSegStages - 1) / kSegStages;
+    const bool magic = stages <= (1 << 22) / (16 * kStageK);
     for (int seg = 0; seg < nseg; ++seg) {
       int go = 1;
       if (lane == 0) go = mbar_wait_sleep(acc_full, (uint32_t)seg & 1u, 3, abort_flag, err) && !*abort_flag;
@@ -291,17 +327,36 @@ fp4_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       for (int b = half; b < CT / 8; b += 2) {
         uint32_t v[56];
         tmem_ld56(tl + (uint32_t)(56 * b), v);
-        if ((int64_t)row_block * 128 < nrows) {
+        if ((int64_t)row_block * 128 >= nrows) continue;
+        const int64_t j0 = (int64_t)bt * CT + 8 * b;
+        if constexpr (kMode == kProduct) {
+          float* D = static_cast<float*>(Dv);
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            const int64_t j = (int64_t)bt * CT + 8 * b + c;
-            long long t = 0;
-#pragma unroll
-            for (int d = kDigits - 1; d >= 0; --d)
-              t = 13 * t + (long long)__float2int_rn(2.0f * __uint_as_float(v[7 * c + d]));
-            const float x = __ll2float_rn(t) * __ldg(descale + j);
-            float* o = D + j * ldd + r;
+            const float x = __ll2float_rn(combine_digits(v + 7 * c, magic)) * __ldg(descale + j0 + c);
+            float* o = D + (j0 + c) * ldd + r;
             *o = seg == 0 ? x : *o + x;
+          }
+        } else if constexpr (kMode == kSums) {
+          long long* D = static_cast<long long*>(Dv);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const long long t = combine_digits(v + 7 * c, magic);
+            long long* o = D + (j0 + c) * ldd + r;
+            *o = seg == 0 ? t : *o + t;
+          }
+        } else {  // one segment only (fp4_syrk checks)
+          float* K = static_cast<float*>(Dv);
+          const long long ar = r < sy.n ? sy.shift[r] : 0;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const int64_t cc = j0 + c;
+            if (cc <= r && cc < nrows) {
+              const long long t = combine_digits(v + 7 * c, magic) - ar - __ldg(sy.shift + (cc < sy.n ? cc : 0)) + sy.c0;
+              const float x = r < sy.n ? __ll2float_rn(t) * sy.scale : 0.0f;
+              K[r * ldd + cc] = x;
+              K[cc * ldd + r] = x;
+            }
           }
         }
       }
@@ -332,16 +387,17 @@ bool fp4_map(CUtensorMap* m, const void* base, int64_t bytes, uint32_t box_rows)
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int CT, int S>
-cudaError_t launch_fp4(const CUtensorMap& a, const CUtensorMap& b, int stages, int64_t rows, int ncolt, float* D,
-                       int64_t ldd, const float* descale, int* err, cudaStream_t s) {
-  auto k = fp4_gemm_kernel<CT, S>;
+// ntiles tiles of 256 rows x CT columns, column tiles (ncolt) fastest.
+template <int CT, int S, int kMode>
+cudaError_t launch_fp4(const CUtensorMap& a, const CUtensorMap& b, int stages, int64_t rows, int64_t ntiles, int ncolt,
+                       void* D, int64_t ldd, const float* descale, const SyrkArgs& sy, int* err, cudaStream_t s) {
+  auto k = fp4_gemm_kernel<CT, S, kMode>;
   constexpr size_t sm = (size_t)S * (kAStage + 336 * CT) + 128 + 256;
   static_assert(sm <= 232448 && 2 * S + 4 <= 31, "stage ring and barriers fit the CTA's shared memory");
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * ((rows + 255) / 256) * ncolt));
+  cfg.gridDim = dim3((unsigned)(2 * ntiles));
   cfg.blockDim = dim3(kFp4Threads);
   cfg.dynamicSmemBytes = sm;
   cfg.stream = s;
@@ -352,7 +408,7 @@ cudaError_t launch_fp4(const CUtensorMap& a, const CUtensorMap& b, int stages, i
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, k, a, b, stages, ncolt, D, ldd, rows, descale, err);
+  e = cudaLaunchKernelEx(&cfg, k, a, b, stages, ncolt, D, ldd, rows, descale, sy, err);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
@@ -408,7 +464,7 @@ __global__ void fp4_gbuild_sm_kernel(const uint8_t* __restrict__ codes, int64_t 
     uint8_t v = 0xFF;  // no copies
     if (mk < m && off < pitch) v = codes[mk * pitch + off];
     sc[mm][b] = v;
-    if (b == 0) sf[mm] = mk < m ? (uint8_t)(2 * fill[mk]) : 0;
+    if (b == 0) sf[mm] = fill && mk < m ? (uint8_t)(2 * fill[mk]) : 0;  // no fill: no missing calls
   }
   __syncthreads();
   for (int t = threadIdx.x; t < kAStage / 16; t += blockDim.x) {
@@ -821,11 +877,12 @@ static cudaError_t fp4_gemm(const void* G, int64_t rows, int64_t k, const void* 
   int* err = tc_error_flag();
   if (!err) return cudaErrorInvalidValue;
   const int nt = (int)(ncols / ct);
+  const int64_t tiles = (rows + 255) / 256 * nt;
   switch (ct) {
-    case 16: return launch_fp4<16, 6>(a, b, stages, rows, nt, D, ldd, descale, err, s);
-    case 32: return launch_fp4<32, 4>(a, b, stages, rows, nt, D, ldd, descale, err, s);
-    case 48: return launch_fp4<48, 7>(a, b, stages, rows, nt, D, ldd, descale, err, s);
-    case 64: return launch_fp4<64, 6>(a, b, stages, rows, nt, D, ldd, descale, err, s);
+    case 16: return launch_fp4<16, 6, kProduct>(a, b, stages, rows, tiles, nt, D, ldd, descale, {}, err, s);
+    case 32: return launch_fp4<32, 4, kProduct>(a, b, stages, rows, tiles, nt, D, ldd, descale, {}, err, s);
+    case 48: return launch_fp4<48, 7, kProduct>(a, b, stages, rows, tiles, nt, D, ldd, descale, {}, err, s);
+    case 64: return launch_fp4<64, 6, kProduct>(a, b, stages, rows, tiles, nt, D, ldd, descale, {}, err, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -861,6 +918,198 @@ cudaError_t fp4_product(const void* Gmm, const void* Gsm, const float* Pf, int64
                                                                     w.part, nblk, nt, winv, Yf);
   *launches = max_w > 0 ? 8 : 7;
   return cudaGetLastError();
+}
+
+// ----------------------------------------------------------------------------------- the GRM
+// K = Z Z' / M from the packed GRM genotypes, z = (g - 2p) / sd:
+//
+//   M K_ij = sum_m D_m g_im g_jm - a_i - a_j + c0,  D = 1/sd^2,  a_i = sum_m 2p_m D_m g_im,  c0 = sum_m 4p_m^2 D_m
+//
+// with D_m fixed to integers (2 D_m <= 2^24).  The rows of B are samples: element m of row j is D_m g_jm, one of
+// 0, D_m, 2 D_m, in base-13 digits; the sums are exact, and so is the subtraction of a_i and a_j, which cancels
+// most of them: only D's rounding (2^-25 of its largest value) and the entry's own rounding to FP32 remain.
+// Against split-BF16's four products (off-diagonal error 4e-8 of entries of RMS 2.6e-3 at 100k x 150k, and row
+// sums off by n times its bias) this takes seven FP4 products, 1.2 BF16 ones' tensor time.
+namespace {
+
+constexpr int kSyrkTile = 64;
+
+// Digits of D_m g_jm for a column tile of 64 samples and one stage of 192 markers: thread = (sample, chunk of 32
+// markers), its masks (one copy, two copies) applied to the stage's digit words.
+// words: [stage][digit][24 groups of 8 markers] of (codes of D, codes of 2 D)
+__global__ void __launch_bounds__(384)
+fp4_syrk_digits_kernel(const uint8_t* __restrict__ packed, int64_t pitch, int64_t m, int64_t n, int stages,
+                       const uint2* __restrict__ words, uint8_t* __restrict__ out) {
+  __shared__ uint8_t sc[kStageK][17];
+  __shared__ uint2 sw[kDigits * 24];
+  const int ks = blockIdx.x;
+  const int64_t tile = blockIdx.y;
+  for (int t = threadIdx.x; t < kStageK * 16; t += blockDim.x) {
+    const int mm = t >> 4, b = t & 15;
+    const int64_t mk = (int64_t)ks * kStageK + mm, off = tile * 16 + b;
+    sc[mm][b] = mk < m && off < pitch ? packed[mk * pitch + off] : 0xFF;
+  }
+  for (int t = threadIdx.x; t < kDigits * 24; t += blockDim.x) sw[t] = words[(int64_t)ks * (kDigits * 24) + t];
+  __syncthreads();
+  const int j = threadIdx.x & 63, chunk = threadIdx.x >> 6;
+  const bool live = tile * 64 + j < n;
+  uint32_t m1[4], m2[4];
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    uint32_t a = 0, b = 0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const uint32_t f = (sc[chunk * 32 + 8 * w + e][j >> 2] >> (2 * (j & 3))) & 3u;
+      a |= (f == 2u ? 15u : 0u) << (4 * e);
+      b |= (f == 0u ? 15u : 0u) << (4 * e);
+    }
+    m1[w] = live ? a : 0u;
+    m2[w] = live ? b : 0u;
+  }
+  const DigitTile dt{kSyrkTile, stages};
+  const DigitColumn dc = digit_column(dt, j);
+  uint8_t* o = out + tile * (int64_t)stages * (672 * kSyrkTile) + (int64_t)ks * (672 * kSyrkTile) + chunk * 128;
+#pragma unroll
+  for (int d = 0; d < kDigits; ++d) {
+    uint32_t x[4];
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const uint2 c = sw[d * 24 + chunk * 4 + w];
+      x[w] = (c.x & m1[w]) | (c.y & m2[w]);
+    }
+    const int r = dc.r + d, rank = r >= dc.hn ? 1 : 0, row = 112 * dc.h + r - rank * dc.hn;
+    *reinterpret_cast<uint4*>(o + rank * (336 * kSyrkTile) + (row >> 3) * kGroupStage + (row & 7) * 16) =
+        make_uint4(x[0], x[1], x[2], x[3]);
+  }
+}
+
+// The two columns of 2p_m D_m 2^16 = hi 2^18 + lo as digits of a 16-column tile (the others zero).
+__global__ void fp4_shift_digits_kernel(const int2* __restrict__ hilo, int64_t m, int stages, uint8_t* __restrict__ out) {
+  const int64_t k = 8 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+  if (k >= (int64_t)stages * kStageK) return;
+  const DigitTile dt{16, stages};
+  for (int j = 0; j < 16; ++j) {
+    int32_t q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      q[i] = 0;
+      if (j < 2 && k + i < m) q[i] = j == 0 ? hilo[k + i].x : hilo[k + i].y;
+    }
+    store_digits(out, dt, j, k, q);
+  }
+}
+
+// a_i = (hi_i 2^18 + lo_i) / 2^16, rounded (the shifted sum stays below 2^62)
+__global__ void fp4_shift_kernel(const long long* __restrict__ sums, int64_t ld, int64_t n, long long* __restrict__ shift) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  shift[i] = ((sums[i] << 18) + sums[ld + i] + (1ll << 15)) >> 16;
+}
+
+}  // namespace
+
+// Bytes of a build's scratch (see fp4_syrk), and whether D's range lets integers of 24 bits hold it: the markers
+// of the smallest D then keep an error of 2^-25 ``range`` relative, at most that of the other builds' genotypes.
+Fp4SyrkPlan fp4_syrk_plan(const double* weight, int64_t m, int64_t np, double range) {
+  Fp4SyrkPlan p;
+  double lo = 1e300, hi = 0.0;
+  for (int64_t i = 0; i < m; ++i) {
+    const double d = weight[i];
+    if (d > 0.0) {
+      lo = d < lo ? d : lo;
+      hi = d > hi ? d : hi;
+    }
+  }
+  if (m <= 0 || !(hi > 0.0) || !(hi < 1e30) || hi > range * lo || fp4_stages(m) > kSegStages) return p;
+  int e = 0;
+  frexp(hi, &e);  // hi < 2^e
+  p.exponent = 23 - e;
+  p.ok = true;
+  const int64_t stages = fp4_stages(m);
+  auto add = [&](int64_t bytes) {
+    const int64_t at = p.bytes;
+    p.bytes += round_up(bytes, 256);
+    return at;
+  };
+  p.off_a = add(fp4_matrix_bytes(np, m));
+  p.off_b = add(round_up(np, kSyrkTile) * stages * 672);
+  p.off_shift_b = add(16 * stages * 672);
+  p.off_sums = add(16 * np * 8);
+  p.off_shift = add(np * 8);
+  p.off_words = add(stages * kDigits * 24 * 8);
+  p.off_hilo = add(m * 8);
+  // lower-triangle tiles: groups of 8 row tiles (256 rows) sweep the column tiles together, so the pairs
+  // resident at one time share a few panels of either operand in L2
+  const int64_t nrt = (np + 255) / 256;
+  for (int64_t g0 = 0; g0 < nrt; g0 += 8) {
+    const int64_t g1 = g0 + 8 < nrt ? g0 + 8 : nrt;
+    for (int64_t bt = 0; bt * kSyrkTile < np && bt * kSyrkTile < g1 * 256; ++bt)
+      for (int64_t rt = g0; rt < g1; ++rt)
+        if (bt * kSyrkTile < rt * 256 + 256) {
+          p.tiles.push_back((int32_t)rt);
+          p.tiles.push_back((int32_t)bt);
+        }
+  }
+  p.off_tiles = add((int64_t)p.tiles.size() * 4);
+  return p;
+}
+
+// K = (1/m) sum_m weight_m (g_i - centre_m) (g_j - centre_m) (np x np, FP32, both triangles) from packed
+// genotypes (m x pitch bytes), in the plan's scratch.  Returns after the work has run.
+cudaError_t fp4_syrk(const Fp4SyrkPlan& p, void* scratch, const uint8_t* packed, int64_t pitch, const double* weight,
+                     const double* centre, int64_t m, int64_t n, int64_t np, float* K, cudaStream_t s) {
+  uint8_t* base = static_cast<uint8_t*>(scratch);
+  const int stages = fp4_stages(m);
+  // host tables: D_m's digit words, (hi, lo) of 2p_m D_m 2^16, c0
+  std::vector<uint32_t> words((size_t)stages * kDigits * 24 * 2, 0u);
+  std::vector<int32_t> hilo((size_t)m * 2);
+  double c0 = 0.0;
+  for (int64_t i = 0; i < m; ++i) {
+    const double two_p = centre[i];
+    const int32_t D = (int32_t)std::llrint(std::ldexp(weight[i], p.exponent));
+    const uint32_t c1 = digit_codes(D), c2 = digit_codes(2 * D);
+    const int64_t ks = i / kStageK, g = (i % kStageK) / 8, e = i % 8;
+    for (int t = 0; t < kDigits; ++t) {
+      uint32_t* w = &words[((size_t)(ks * kDigits + t) * 24 + g) * 2];
+      w[0] |= ((c1 >> (4 * t)) & 15u) << (4 * e);
+      w[1] |= ((c2 >> (4 * t)) & 15u) << (4 * e);
+    }
+    const long long h = std::llrint(std::ldexp((double)D * two_p, 16));
+    hilo[2 * i] = (int32_t)(h >> 18);
+    hilo[2 * i + 1] = (int32_t)(h & ((1 << 18) - 1));
+    c0 += (double)D * two_p * two_p;
+  }
+  cudaError_t e = cudaMemcpyAsync(base + p.off_words, words.data(), words.size() * 4, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(base + p.off_hilo, hilo.data(), hilo.size() * 4, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(base + p.off_tiles, p.tiles.data(), p.tiles.size() * 4, cudaMemcpyHostToDevice, s);
+  if (e != cudaSuccess) return e;
+  const int64_t rs = (np + 255) / 256 * 2;
+  fp4_gbuild_sm_kernel<<<dim3((unsigned)stages, (unsigned)rs), 256, 0, s>>>(
+      packed, pitch, nullptr, m, n, stages, reinterpret_cast<uint4*>(base + p.off_a));
+  const int64_t nbt = (np + kSyrkTile - 1) / kSyrkTile;
+  fp4_syrk_digits_kernel<<<dim3((unsigned)stages, (unsigned)nbt), 384, 0, s>>>(
+      packed, pitch, m, n, stages, reinterpret_cast<const uint2*>(base + p.off_words), base + p.off_b);
+  fp4_shift_digits_kernel<<<(unsigned)((stages * (kStageK / 8) + 127) / 128), 128, 0, s>>>(
+      reinterpret_cast<const int2*>(base + p.off_hilo), m, stages, base + p.off_shift_b);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  CUtensorMap a, b, bs;
+  int* err = tc_error_flag();
+  if (!err || !fp4_map(&a, base + p.off_a, fp4_matrix_bytes(np, m), kAStage / kMapRow) ||
+      !fp4_map(&b, base + p.off_b, round_up(np, kSyrkTile) * (int64_t)stages * 672, 336 * kSyrkTile / kMapRow) ||
+      !fp4_map(&bs, base + p.off_shift_b, 16 * (int64_t)stages * 672, 336 * 16 / kMapRow))
+    return cudaErrorInvalidValue;
+  long long* sums = reinterpret_cast<long long*>(base + p.off_sums);
+  long long* shift = reinterpret_cast<long long*>(base + p.off_shift);
+  e = launch_fp4<16, 6, kSums>(a, bs, stages, np, (np + 255) / 256, 1, sums, np, nullptr, {}, err, s);
+  if (e != cudaSuccess) return e;
+  fp4_shift_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(sums, np, n, shift);
+  const SyrkArgs sy{reinterpret_cast<const int2*>(base + p.off_tiles), shift, std::llrint(c0),
+                    (float)(std::ldexp(1.0, -p.exponent) / (double)m), n};
+  e = launch_fp4<kSyrkTile, 6, kSyrk>(a, b, stages, np, (int64_t)p.tiles.size() / 2, 1, K, np, nullptr, sy, err, s);
+  if (e != cudaSuccess) return e;
+  return tc_check_error(s);
 }
 
 }  // namespace sg

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from oracle import aireml, plink
-from saigegpu import MV_FP32_SIMT, MV_SUBSET_EXACT, synth
+from saigegpu import GRM_BF16X3_TC, GRM_FP32_SIMT, MV_FP32_SIMT, MV_SUBSET_EXACT, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -101,3 +101,40 @@ def test_refused_memory_falls_back(gpu_ctx):
             if budget is None:
                 np.testing.assert_array_equal(out[1], ctx.grm_matmul(b).astype(np.float32))
     np.testing.assert_allclose(out[0], out[1], rtol=0, atol=6e-5 * np.abs(out[0]).max())
+
+
+@pytest.mark.parametrize("precision,tol", [(GRM_FP32_SIMT, 4 * 2.0 ** -23), (GRM_BF16X3_TC, 2.0 ** -16)])
+@pytest.mark.parametrize("n,m", [(33, 40), (64, 192), (65, 193), (256, 700), (300, 191), (641, 1500)])
+def test_grm_matches_fp64_at_tile_edges(gpu_ctx, n, m, precision, tol):
+    """Every entry of K against the FP64 GRM.  FP32: its own rounding (2^-24) and the oracle's, whose
+    standardised genotypes are FP32 values (2^-23 of each term).  Split BF16: genotypes of 16 bits
+    (2^-17 of each of a term's two factors)."""
+    bed, _ = synth.synth_bed(900 + n, n, m, 0.02)
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    ref = aireml.DenseGRM(plink.setgeno(bed, n, m, np.arange(1, n + 1), np.ones(n, bool), 0.01, 0.15)).K
+    ctx.grm_build(precision)
+    K = ctx.grm_get()
+    assert np.abs(K - ref).max() < tol * np.abs(ref).max()
+    np.testing.assert_array_equal(K, K.T)
+    ctx.grm_build(precision)  # over the resident K
+    np.testing.assert_array_equal(ctx.grm_get(), K)
+
+
+@pytest.mark.parametrize("precision,tol", [(GRM_FP32_SIMT, 2e-6), (GRM_BF16X3_TC, 2e-5)])
+def test_grm_of_a_wide_frequency_range_takes_the_other_builds(gpu_ctx, precision, tol):
+    """A marker carried once among 3,000 samples: 1/sd^2 spans a factor of 1,500."""
+    n, m = 3000, 400
+    bed, _ = synth.synth_bed(77, n, m, 0.0)
+    raw = np.frombuffer(bed, np.uint8).copy()
+    nb = (n + 3) // 4
+    raw[3:3 + nb] = 0xFF
+    raw[3] = 0xFE  # the first sample of the first marker has one copy
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(raw, n, m, min_maf=0.0)
+    g = plink.setgeno(raw.tobytes(), n, m, np.arange(1, n + 1), np.ones(n, bool), 0.0, 0.15)
+    ref = aireml.DenseGRM(g).K
+    ctx.grm_build(precision)
+    assert np.abs(ctx.grm_get() - ref).max() < tol * np.abs(ref).max()
