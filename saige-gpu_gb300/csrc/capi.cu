@@ -832,6 +832,39 @@ static int setgeno_core(sg_ctx* c, const uint8_t* raw, int64_t raw_pitch, int64_
   return SG_OK;
 }
 
+// Bytes of a re-pitching copy's staging buffer on the device.
+constexpr int64_t kBedStage = int64_t(64) << 20;
+
+// A .bed body in host memory to pitched rows: contiguous copies of up to 64 MB of whole rows, each re-pitched by
+// a kernel (or, with no memory for the staging buffer, one pitched copy).
+static int bed_upload(sg_ctx* c, const uint8_t* body, int64_t nb, int64_t m, int64_t n_fam, uint8_t* raw,
+                      int64_t raw_pitch) {
+  if (m == 0) return SG_OK;
+  const int64_t rows = std::min(m, std::max<int64_t>(1, kBedStage / nb));
+  uint8_t* flat = nullptr;
+  const std::string err = c->err;
+  if (dev_alloc_t(c, &flat, (size_t)(rows * nb + 16)) != SG_OK) {
+    c->err = err;
+    SG_CUDA(c, cudaMemsetAsync(raw, 0, raw_pitch * m, c->stream));
+    SG_CUDA(c, cudaMemcpy2DAsync(raw, raw_pitch, body, nb, nb, m, cudaMemcpyHostToDevice, c->stream));
+    return SG_OK;
+  }
+  cudaError_t e = cudaSuccess;
+  for (int64_t r = 0; r < m && e == cudaSuccess; r += rows) {
+    const int64_t k = std::min(rows, m - r);
+    e = cudaMemcpyAsync(flat, body + r * nb, k * nb, cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) {
+      launch_bed_pitch(flat, flat + k * nb, nb, k, n_fam, raw + r * raw_pitch, raw_pitch, c->stream);
+      c->launches += 1;
+      e = cudaGetLastError();
+    }
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  dev_free(c, flat);
+  if (e != cudaSuccess) return set_err(c, SG_ERR_CUDA, "genotype upload: %s", cudaGetErrorString(e));
+  return SG_OK;
+}
+
 static int setgeno_common(sg_ctx* c, const uint8_t* bed, bool on_device, uint64_t bed_len,
                           int64_t n_fam, int64_t m_bim, const int32_t* sub_1based, int64_t n_sub,
                           const uint8_t* pheno_mask, float min_maf, float max_missing,
@@ -857,11 +890,16 @@ static int setgeno_common(sg_ctx* c, const uint8_t* bed, bool on_device, uint64_
   const int64_t raw_pitch = round_up(std::max<int64_t>(nb, 1), kPitchAlign);
   uint8_t* raw = nullptr;
   SG_TRY(dev_alloc_t(c, &raw, (size_t)std::max<int64_t>(raw_pitch * m_bim, 16)));
-  SG_CUDA(c, cudaMemsetAsync(raw, 0, raw_pitch * std::max<int64_t>(m_bim, 1), c->stream));
-  if (m_bim)
-    SG_CUDA(c, cudaMemcpy2DAsync(raw, raw_pitch, bed + 3, nb, nb, m_bim,
-                                 on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                                 c->stream));
+  if (on_device) {
+    launch_bed_pitch(bed + 3, bed + 3 + nb * m_bim, nb, m_bim, n_fam, raw, raw_pitch, c->stream);
+    SG_LAUNCHED(c, m_bim ? 1 : 0);
+  } else {
+    const int rc_up = bed_upload(c, bed + 3, nb, m_bim, n_fam, raw, raw_pitch);
+    if (rc_up != SG_OK) {
+      dev_free(c, raw);
+      return rc_up;
+    }
+  }
   int rc = setgeno_core(c, raw, raw_pitch, n_fam, m_bim, sub_1based, n_sub, pheno_mask, min_maf,
                         max_missing, vr_markers, n_vr, min_mac_vr, is_var_ratio, is_diag_one);
   cudaStreamSynchronize(c->stream);
@@ -967,8 +1005,25 @@ extern "C" int sg_get_vr_markers(sg_ctx* c, float* freq, int32_t* mac, int32_t* 
 extern "C" int sg_get_packed_geno(sg_ctx* c, uint8_t* out) {
   NEED_GENO(c);
   const int64_t nb = (c->nn + 3) / 4;
-  if (c->m_qc)
+  if (c->m_qc == 0) return SG_OK;
+  const int64_t rows = std::min(c->m_qc, std::max<int64_t>(1, kBedStage / nb));
+  uint8_t* flat = nullptr;
+  const std::string err = c->err;
+  if (nb == c->pitch || dev_alloc_t(c, &flat, (size_t)(rows * nb + 16)) != SG_OK) {
+    c->err = err;
     SG_CUDA(c, cudaMemcpy2D(out, nb, c->d_packed, c->pitch, nb, c->m_qc, cudaMemcpyDeviceToHost));
+    return SG_OK;
+  }
+  cudaError_t e = cudaSuccess;
+  for (int64_t r = 0; r < c->m_qc && e == cudaSuccess; r += rows) {
+    const int64_t k = std::min(rows, c->m_qc - r);
+    launch_bed_unpitch(c->d_packed + r * c->pitch, c->pitch, nb, k, flat, c->stream);
+    c->launches += 1;
+    e = cudaMemcpyAsync(out + r * nb, flat, k * nb, cudaMemcpyDeviceToHost, c->stream);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  dev_free(c, flat);
+  if (e != cudaSuccess) return set_err(c, SG_ERR_CUDA, "genotype read-back: %s", cudaGetErrorString(e));
   return SG_OK;
 }
 

@@ -111,6 +111,69 @@ void launch_marker_qc(const uint8_t* raw, int64_t raw_pitch, int64_t m, int64_t 
 }
 
 // ----------------------------------------------------------------------------
+// Rows of nb bytes back to back (a .bed body, at any alignment) to and from rows of ``pitch`` bytes.  A
+// copy engine moves such rows one by one (5,003-byte rows: ~60 ms a way for 150 MB of pageable memory); a
+// contiguous copy of them takes 0.9 ms, so the bytes cross the bus contiguously and a kernel re-pitches them
+// in HBM.  Bounded by HBM; setgeno of that image and its read-back went from 146 to 14.7 ms, most of it now
+// the page faults of the caller's fresh output array.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t load_u32_at(const uint8_t* a, const uint8_t* end) {
+  const uintptr_t u = reinterpret_cast<uintptr_t>(a);
+  const uint32_t* p = reinterpret_cast<const uint32_t*>(u & ~uintptr_t(3));
+  const unsigned sh = 8u * (unsigned)(u & 3);
+  if (reinterpret_cast<const uint8_t*>(p + 2) <= end) return __funnelshift_r(p[0], p[1], sh);
+  uint32_t v = 0;  // the last bytes one by one: nothing past the end is read
+  for (int i = 0; i < 4; ++i)
+    if (a + i < end) v |= (uint32_t)a[i] << (8 * i);
+  return v;
+}
+
+// bytes past nb and the fields of samples past n are zero
+__global__ void bed_pitch_kernel(const uint8_t* __restrict__ src, const uint8_t* src_end, int64_t nb, int64_t rows,
+                                 int64_t n, uint32_t* __restrict__ out, int64_t pitch) {
+  const int64_t wpr = pitch / 4;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rows * wpr; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = t / wpr, w = t - r * wpr;
+    uint32_t v = 0;
+    if (4 * w < nb) {
+      v = load_u32_at(src + r * nb + 4 * w, src_end);
+      const int64_t left = n - 16 * w;  // samples from this word on
+      if (left < 16) v &= (1u << (2 * left)) - 1u;
+    }
+    out[t] = v;
+  }
+}
+
+__global__ void bed_unpitch_kernel(const uint8_t* __restrict__ in, int64_t pitch, int64_t nb, int64_t rows,
+                                   uint32_t* __restrict__ out) {
+  const int64_t total = rows * nb, words = (total + 3) / 4;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < words; t += (int64_t)gridDim.x * blockDim.x) {
+    int64_t r = 4 * t / nb, b = 4 * t - r * nb;
+    uint32_t v = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (4 * t + i < total) v |= (uint32_t)in[r * pitch + b] << (8 * i);
+      if (++b == nb) {
+        b = 0;
+        ++r;
+      }
+    }
+    out[t] = v;
+  }
+}
+
+void launch_bed_pitch(const uint8_t* src, const uint8_t* src_end, int64_t nb, int64_t rows, int64_t n, uint8_t* out,
+                      int64_t pitch, cudaStream_t s) {
+  if (rows == 0) return;
+  bed_pitch_kernel<<<152 * 16, 256, 0, s>>>(src, src_end, nb, rows, n, reinterpret_cast<uint32_t*>(out), pitch);
+}
+
+void launch_bed_unpitch(const uint8_t* in, int64_t pitch, int64_t nb, int64_t rows, uint8_t* out, cudaStream_t s) {
+  if (rows == 0) return;
+  bed_unpitch_kernel<<<152 * 16, 256, 0, s>>>(in, pitch, nb, rows, reinterpret_cast<uint32_t*>(out));
+}
+
+// ----------------------------------------------------------------------------
 // Re-pack (FIT.cpp:551-575): for output marker j (source marker src_marker[j]),
 // sample k takes the source field of sample sub0[k]; a missing field (01)
 // becomes the code of the fill genotype.  The reference's re-pack codes

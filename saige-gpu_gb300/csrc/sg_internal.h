@@ -42,6 +42,12 @@ void launch_marker_qc(const uint8_t* raw, int64_t raw_pitch, int64_t m, int64_t 
                       const uint32_t* maskbits, int64_t nn, float min_maf, float max_miss,
                       const uint8_t* vr_flag, float min_mac_vr, float max_mac_vr, int is_var_ratio,
                       MarkerQC* out, cudaStream_t s);
+// rows of nb bytes back to back (src up to src_end, any alignment) to rows of pitch bytes (a multiple of
+// 16), bytes past nb and samples past n zero; and rows of pitch bytes to rows of nb back to back (out: rows
+// * nb bytes rounded up to 4)
+void launch_bed_pitch(const uint8_t* src, const uint8_t* src_end, int64_t nb, int64_t rows, int64_t n, uint8_t* out,
+                      int64_t pitch, cudaStream_t s);
+void launch_bed_unpitch(const uint8_t* in, int64_t pitch, int64_t nb, int64_t rows, uint8_t* out, cudaStream_t s);
 // qc == nullptr keeps missing calls (code 01) instead of writing the fill genotype's code
 void launch_repack(const uint8_t* raw, int64_t raw_pitch, const int32_t* src_marker,
                    const MarkerQC* qc, int64_t m_out, const int32_t* sub0, int64_t nn,

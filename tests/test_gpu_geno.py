@@ -73,3 +73,19 @@ def test_bad_inputs_raise(gpu_ctx):
         gpu_ctx.setgeno(bed, 8, 4, np.array([0, 1], np.int32))
     with pytest.raises(SaigeGpuError):
         gpu_ctx.setgeno(bed[:-1], 8, 4)
+
+
+@pytest.mark.parametrize("n,m", [(1, 3), (4, 2), (5, 7), (61, 5), (64, 9), (65, 4), (4099, 70000)])
+def test_host_and_device_images_give_the_same_genotypes(gpu_ctx, n, m):
+    """A .bed image in host memory (contiguous copies re-pitched on the device, 64 MB of rows at a time: the
+    last size takes two) against the same image on the device, and small ones against the oracle's re-pack."""
+    ptr, ln = gpu_ctx.synth_bed(7 + n, n, m, 0.1)
+    host = gpu_ctx.synth_bed_to_host(ln)
+    gpu_ctx.setgeno_device(ptr, ln, n, m, min_maf=0.0, max_missing=1.0)
+    packed, diag = gpu_ctx.packed_geno(), gpu_ctx.grm_diag_f32()
+    gpu_ctx.setgeno(host, n, m, min_maf=0.0, max_missing=1.0)
+    np.testing.assert_array_equal(gpu_ctx.packed_geno(), packed)
+    np.testing.assert_array_equal(gpu_ctx.grm_diag_f32(), diag)
+    if n * m < 10000:
+        o = plink.setgeno(host.tobytes(), n, m, np.arange(1, n + 1), np.ones(n, bool), 0.0, 1.0)
+        np.testing.assert_array_equal(packed, plink.pack_codes(o.codes))
