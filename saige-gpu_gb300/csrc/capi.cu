@@ -185,7 +185,8 @@ struct Engine {
   double* spart = nullptr;        // column partials: cap_cols x max(blocks over np, over mg)
   float* smax = nullptr;          // FP16 / E4M3 form: column block maxima, as spart
   float* sscale = nullptr;        //   and the columns' power-of-two scales s1, s2 (2 x cap_cols)
-  bool digits = false;            // products on the FP4 pipe (the FP32 drop-ins, DigitsScope)
+  bool list_up = false;           // the step's active columns are on the device
+  int64_t fp32_cols = 0;          // > 0: a drop-in that returns FP32 runs, with steps of up to so many columns
   Fp4Scratch f4;
   float* sdiag_part[kSetupStreams] = {};  // per-chunk partial sums of a subset's diagonal, per set-up stream
 
@@ -271,6 +272,14 @@ struct sg_ctx {
   // the same values in E2M1 for the FP32 drop-ins' products (k_fp4.cu), built at the first of them
   void* d_G4 = nullptr;
   bool g4_refused = false;  // no memory for it: those products run as the others
+  // the GRM markers' genotypes alike, with the one slot record of the whole cohort: the FP32 drop-ins'
+  // products on a resident GRM, where that reads fewer bytes than K
+  void* d_Gk = nullptr;
+  SubsetSlot* d_gk_slot = nullptr;
+  double* d_gk_p2d = nullptr;
+  float *d_gk_dp = nullptr, *d_gk_p2 = nullptr;
+  bool gk_refused = false;
+  bool k_exact = false;     // K holds the FP32-class GRM (not the single-product BF16 one)
   // synthetic bed image
   uint8_t* d_synth = nullptr;
   uint64_t synth_len = 0;
@@ -484,6 +493,7 @@ static void engine_free(sg_ctx* c);
 
 static int ensure_g(sg_ctx* c, int form);
 static void free_g(sg_ctx* c);
+static void free_gk(sg_ctx* c);
 
 // the subset-exact engines (BF16 products, or FP16 high / E4M3 low)
 static bool exact_mode(int mode) { return mode == SG_MV_SUBSET_EXACT || mode == SG_MV_SUBSET_EXACT_F8; }
@@ -517,6 +527,7 @@ extern "C" int sg_set_matvec_mode(sg_ctx* c, int mode) {
     std::fill(c->eng.ph_set.begin(), c->eng.ph_set.end(), 0);
   }
   if (exact_mode(mode)) {
+    free_gk(c);
     SG_TRY(ensure_k_split(c, false));
     SG_TRY(ensure_k_bf16(c, false));
     return ensure_g(c, mode == SG_MV_SUBSET_EXACT_F8 ? 1 : 0);
@@ -524,6 +535,10 @@ extern "C" int sg_set_matvec_mode(sg_ctx* c, int mode) {
   if (was_exact) {  // the genotype matrix (2 bytes per sample and marker, twice) leaves HBM
     SG_TRY(sync(c));
     free_g(c);
+  }
+  if (mode != SG_MV_BF16X3_TC && c->d_Gk) {
+    SG_TRY(sync(c));
+    free_gk(c);
   }
   if (!c->have_grm) return SG_OK;
   SG_TRY(ensure_k_split(c, mode == SG_MV_TF32X3_TC));
@@ -664,6 +679,7 @@ static void free_geno(sg_ctx* c) {
   c->k_split = false;
   dev_free(c, c->d_Kb);
   c->d_Kb = nullptr;
+  free_gk(c);
   dev_free_t(c, c->d_diag);
   dev_free_t(c, c->d_diag32);
   dev_free_t(c, c->d_codes);
@@ -1115,7 +1131,9 @@ extern "C" int sg_grm_build(sg_ctx* c, int precision) {
   c->d_Kb = nullptr;
   engine_free(c);
   loco_free(c);
+  free_gk(c);
   c->have_grm = false;
+  c->k_exact = precision != SG_GRM_BF16_TC;
   c->np = np;
   if (!c->d_K) SG_TRY(dev_alloc_t(c, &c->d_K, (size_t)(np * np)));
   const float scale = 1.0f / (float)c->m_qc;
@@ -1283,6 +1301,16 @@ static cudaError_t d2h(sg_ctx* c, void* dst, const void* src, size_t bytes, cuda
   return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
 }
 
+static void free_gk(sg_ctx* c) {
+  dev_free(c, c->d_Gk);
+  c->d_Gk = nullptr;
+  dev_free_t(c, c->d_gk_slot);
+  dev_free_t(c, c->d_gk_p2d);
+  dev_free_t(c, c->d_gk_dp);
+  dev_free_t(c, c->d_gk_p2);
+  c->gk_refused = false;
+}
+
 static void fp4_free(sg_ctx* c) {
   Fp4Scratch& w = c->eng.f4;
   dev_free(c, w.Vq);
@@ -1292,26 +1320,36 @@ static void fp4_free(sg_ctx* c) {
   w = Fp4Scratch{};
 }
 
-// The E2M1 genotype matrix and the scratch of the FP4 products; false when there is no memory (or
-// budget) for them, and the products then run as the engine's others do.
+// Scratch of the FP4 products over up to mg markers (a multiple of 128).
+static int fp4_scratch(sg_ctx* c, int64_t mg) {
+  Engine& e = c->eng;
+  Fp4Scratch& w = e.f4;
+  if (w.T && w.mg >= mg) return SG_OK;
+  fp4_free(c);
+  const int64_t cap = e.cap_cols + kFp4PadCols, nb = cap * fp4_nblk(e.np, mg);
+  SG_TRY(dev_alloc(c, &w.Vq, (size_t)fp4_digit_bytes(cap, c->nn)));
+  SG_TRY(dev_alloc(c, &w.Tq, (size_t)fp4_digit_bytes(cap, mg)));
+  SG_TRY(dev_alloc_t(c, &w.U, (size_t)(cap * e.np)));
+  SG_TRY(dev_alloc_t(c, &w.part, (size_t)nb));
+  SG_TRY(dev_alloc_t(c, &w.qsum, (size_t)nb));
+  SG_TRY(dev_alloc_t(c, &w.pmax, (size_t)nb));
+  for (float** p : {&w.mean, &w.descale1, &w.descale2}) SG_TRY(dev_alloc_t(c, p, (size_t)cap));
+  SG_TRY(dev_alloc_t(c, &w.T, (size_t)(cap * mg)));
+  w.mg = mg;
+  return SG_OK;
+}
+
+// The E2M1 genotype matrix of the subset-exact engine and the scratch of its FP4 products; false when there is
+// no memory (or budget) for them, and the products then run as the engine's others do.
 static bool fp4_ready(sg_ctx* c) {
   Engine& e = c->eng;
-  if (c->d_G4 && e.f4.T) return true;
+  if (c->d_G4 && e.f4.T && e.f4.mg >= c->mg) return true;
   if (c->g4_refused) return false;
-  const int64_t mm = fp4_matrix_bytes(c->mg, c->nn), cap = e.cap_cols + kFp4PadCols;
-  const int64_t nb = cap * fp4_nblk(e.np, c->mg);
-  Fp4Scratch& w = e.f4;
+  const int64_t mm = fp4_matrix_bytes(c->mg, c->nn);
   const bool build = !c->d_G4;
   auto all = [&]() -> int {
     if (build) SG_TRY(dev_alloc(c, &c->d_G4, (size_t)(mm + fp4_matrix_bytes(e.np, c->m_bim))));
-    SG_TRY(dev_alloc(c, &w.Vq, (size_t)fp4_digit_bytes(cap, c->nn)));
-    SG_TRY(dev_alloc(c, &w.Tq, (size_t)fp4_digit_bytes(cap, c->m_bim)));
-    SG_TRY(dev_alloc_t(c, &w.U, (size_t)(cap * e.np)));
-    SG_TRY(dev_alloc_t(c, &w.part, (size_t)nb));
-    SG_TRY(dev_alloc_t(c, &w.qsum, (size_t)nb));
-    SG_TRY(dev_alloc_t(c, &w.pmax, (size_t)nb));
-    for (float** p : {&w.mean, &w.descale1, &w.descale2}) SG_TRY(dev_alloc_t(c, p, (size_t)cap));
-    return dev_alloc_t(c, &w.T, (size_t)(cap * c->mg));
+    return fp4_scratch(c, c->mg);
   };
   const std::string err = c->err;
   if (all() != SG_OK) {
@@ -1332,15 +1370,86 @@ static bool fp4_ready(sg_ctx* c) {
   return true;
 }
 
-// While it lives, the subset-exact engine's products run on the FP4 pipe (k_fp4.cu).  The drop-ins
-// that return FP32, as the reference's entry points do, hold one; the FP64 interfaces (the engine,
-// sg_pcg_solve, sg_grm_matmul and the batched fits over them) keep the BF16 products, and with them
-// their results bit for bit.
-struct DigitsScope {
+// The same for the cohort's GRM markers, beside a resident K.
+static int fp4_cohort_build(sg_ctx* c) {
+  const int64_t m = c->m_qc, mg = round_up(m, kRowTile), mm = fp4_matrix_bytes(mg, c->nn);
+  SG_TRY(dev_alloc(c, &c->d_Gk, (size_t)(mm + fp4_matrix_bytes(c->np, m))));
+  SG_TRY(dev_alloc_t(c, &c->d_gk_dp, (size_t)mg));
+  SG_TRY(dev_alloc_t(c, &c->d_gk_p2, (size_t)mg));
+  SG_TRY(dev_alloc_t(c, &c->d_gk_p2d, (size_t)mg));
+  SG_TRY(dev_alloc_t(c, &c->d_gk_slot, 1));
+  std::vector<float> dp(mg, 0.0f), p2(mg, 0.0f);
+  std::vector<double> p2d(mg, 0.0);
+  for (int64_t i = 0; i < m; ++i) {
+    dp[i] = (float)((double)c->invstd[i] * (double)c->invstd[i]);
+    p2[i] = 2.0f * c->freq[i];
+    p2d[i] = 2.0 * (double)c->freq[i];
+  }
+  SubsetSlot sl;
+  sl.dprime = c->d_gk_dp;
+  sl.p2 = c->d_gk_p2;
+  sl.p2d = c->d_gk_p2d;
+  sl.flips = nullptr;
+  sl.dfill = nullptr;
+  sl.bits = nullptr;
+  sl.inv_m = 1.0 / (double)m;
+  sl.ns = (double)c->nn;
+  SG_CUDA(c, cudaMemcpyAsync(c->d_gk_dp, dp.data(), mg * 4, cudaMemcpyHostToDevice, c->stream));
+  SG_CUDA(c, cudaMemcpyAsync(c->d_gk_p2, p2.data(), mg * 4, cudaMemcpyHostToDevice, c->stream));
+  SG_CUDA(c, cudaMemcpyAsync(c->d_gk_p2d, p2d.data(), mg * 8, cudaMemcpyHostToDevice, c->stream));
+  SG_CUDA(c, cudaMemcpyAsync(c->d_gk_slot, &sl, sizeof(sl), cudaMemcpyHostToDevice, c->stream));
+  uint8_t* g = static_cast<uint8_t*>(c->d_Gk);
+  launch_fp4_gbuild(c->d_packed, c->pitch, nullptr, m, c->nn, g, g + mm, c->stream);
+  SG_LAUNCHED(c, 2);
+  return sync(c);  // the tables above are on this function's stack
+}
+
+static bool fp4_cohort_ready(sg_ctx* c) {
+  if (c->gk_refused) return false;
+  const std::string err = c->err;
+  const int64_t mg = round_up(c->m_qc, kRowTile);
+  if ((!c->d_Gk && fp4_cohort_build(c) != SG_OK) || fp4_scratch(c, mg) != SG_OK) {
+    fp4_free(c);
+    free_gk(c);
+    c->gk_refused = true;
+    c->err = err;
+    return false;
+  }
+  return true;
+}
+
+// While it lives, products may take the forms below, whose rounding differs from the engines' own.  The drop-ins
+// that return FP32, as the reference's entry points do, hold one; the FP64 interfaces (the engine, sg_pcg_solve,
+// sg_grm_matmul and the batched fits over them) do not, and keep their engine's arithmetic.  cols: the most
+// columns a step of the call has, so that one call's steps all take one form.
+struct Fp32Scope {
   Engine& e;
-  explicit DigitsScope(sg_ctx* c) : e(c->eng) { e.digits = c->mv_mode == SG_MV_SUBSET_EXACT; }
-  ~DigitsScope() { e.digits = false; }
+  Fp32Scope(sg_ctx* c, int64_t cols) : e(c->eng) {
+    if (!e.fp32_cols) e.fp32_cols = cols;
+    else outer = true;  // a drop-in inside another keeps the outer call's form
+  }
+  ~Fp32Scope() {
+    if (!outer) e.fp32_cols = 0;
+  }
+  bool outer = false;
 };
+
+// Forms of a drop-in's product.  Genotypes: exact integers through G on the FP4 pipe (k_fp4.cu) in the
+// subset-exact engine, and in the split-BF16 engine over an FP32-class K where G's two half-byte matrices (n
+// M bytes) are at most 0.6 of K's 4 n^2: K is then read at ~0.55 of the copy rate by the 32-column split GEMM,
+// G at 1.0 with five short kernels beside (n = 20,000, M = 30,000, one column: 0.46 against 0.13 ms).
+// Gemv: FP32 K streamed once per eight columns, in the FP32 engine (measured against its GEMM at the gemv
+// kernel); beyond 16 columns only while K stays near L2's size.
+enum class Fp32Form { kEngine, kGenotypes, kGemv };
+static Fp32Form fp32_form(sg_ctx* c) {
+  const Engine& e = c->eng;
+  if (!e.fp32_cols || c->loco) return Fp32Form::kEngine;
+  if (c->mv_mode == SG_MV_SUBSET_EXACT) return fp4_ready(c) ? Fp32Form::kGenotypes : Fp32Form::kEngine;
+  if (c->mv_mode == SG_MV_BF16X3_TC && c->k_exact && !c->k_split && (double)c->m_qc <= 2.4 * (double)c->nn)
+    return fp4_cohort_ready(c) ? Fp32Form::kGenotypes : Fp32Form::kEngine;
+  if (c->mv_mode == SG_MV_FP32_SIMT && !c->k_split && (e.fp32_cols <= 16 || e.np <= 8192)) return Fp32Form::kGemv;
+  return Fp32Form::kEngine;
+}
 
 static void engine_free(sg_ctx* c) {
   Engine& e = c->eng;
@@ -2192,6 +2301,32 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
   Engine& e = c->eng;
   *used_yf = true;
   *launched = ncols;
+  const Fp32Form form = fp32_form(c);
+  if (form != Fp32Form::kEngine) {
+    const int64_t nact = e.nact;
+    *launched = nact;
+    if (nact == 0) return SG_OK;
+    const bool subset = exact_mode(c->mv_mode);
+    const int ct = form == Fp32Form::kGemv ? 1 : fp4_tile_cols(nact);
+    const int64_t npad = round_up(nact, ct);
+    for (int64_t j = nact; j < npad; ++j) e.h_gcols[j] = -1;
+    SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, npad * 4, cudaMemcpyHostToDevice, c->stream));
+    e.list_up = true;
+    int nl = 1;
+    if (form == Fp32Form::kGemv) {
+      launch_gemv_multi(c->d_K, e.np, e.Pf, e.d_gcols, nact, e.Yf, c->stream);
+    } else {
+      const int64_t m = subset ? c->m_bim : c->m_qc, mg = subset ? c->mg : round_up(m, kRowTile);
+      const uint8_t* g = static_cast<const uint8_t*>(subset ? c->d_G4 : c->d_Gk);
+      const cudaError_t err = fp4_product(g, g + fp4_matrix_bytes(mg, c->nn), e.Pf, e.np, c->nn, mg, m, e.d_gcols, npad, ct,
+                                          e.d_st, subset ? e.d_slots : c->d_gk_slot, e.winv, subset ? e.max_w : 0, e.f4,
+                                          e.Yf, c->stream, &nl);
+      if (err != cudaSuccess) return set_err(c, SG_ERR_CUDA, "tcgen05 genotype GEMM: %s", cudaGetErrorString(err));
+      *launched = npad;
+    }
+    SG_LAUNCHED(c, nl);
+    return SG_OK;
+  }
   if (c->mv_mode == SG_MV_FP64_PLAIN) {
     *used_yf = false;
     if (!e.Yd) SG_TRY(dev_alloc_t(c, &e.Yd, (size_t)(e.cap_cols * e.np)));
@@ -2216,6 +2351,7 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
     const int64_t npad = tc_grmv_padded_cols(round_up(nact, 16), e.cap_cols, e.np, kTilesSplitBF16, c->num_sms);
     for (int64_t j = nact; j < npad; ++j) e.h_gcols[j] = -1;
     SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, npad * 4, cudaMemcpyHostToDevice, c->stream));
+    e.list_up = true;
     uint16_t* ph = static_cast<uint16_t*>(e.Pb);
     launch_split_bf16_gather(e.Pf, e.np, e.d_gcols, npad, ph, ph + half, c->stream);
     c->launches += 1;
@@ -2235,23 +2371,10 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
       return SG_OK;
     }
     const int64_t np = e.np, mg = c->mg;
-    if (e.digits && fp4_ready(c)) {
-      const int ct = fp4_tile_cols(nact);
-      const int64_t npad = round_up(nact, ct);
-      for (int64_t j = nact; j < npad; ++j) e.h_gcols[j] = -1;
-      SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, npad * 4, cudaMemcpyHostToDevice, c->stream));
-      int nl = 0;
-      const uint8_t* g4 = static_cast<const uint8_t*>(c->d_G4);
-      const cudaError_t err = fp4_product(g4, g4 + fp4_matrix_bytes(mg, c->nn), e.Pf, np, c->nn, mg, c->m_bim, e.d_gcols,
-                                          npad, ct, e.d_st, e.d_slots, e.winv, e.max_w, e.f4, e.Yf, c->stream, &nl);
-      if (err != cudaSuccess) return set_err(c, SG_ERR_CUDA, "tcgen05 genotype GEMM: %s", cudaGetErrorString(err));
-      SG_LAUNCHED(c, nl);
-      *launched = npad;
-      return SG_OK;
-    }
     const int64_t npad = tc_grmv_padded_cols(round_up(nact, 32), e.cap_cols, np, kTilesSplitB, c->num_sms);
     for (int64_t j = nact; j < npad; ++j) e.h_gcols[j] = -1;
     SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, npad * 4, cudaMemcpyHostToDevice, c->stream));
+    e.list_up = true;
     const size_t cap = (size_t)e.cap_cols;
     if (!e.Vb) SG_TRY(dev_alloc(c, &e.Vb, cap * np * 4));
     if (!e.Tm) SG_TRY(dev_alloc_t(c, &e.Tm, cap * mg));
@@ -2352,6 +2475,7 @@ static int step_launch(sg_ctx* c) {
   // the step's active columns (host view: admitted columns count as active until their state comes
   // back); the GRM.V compaction and the vector kernels work on this list only
   e.nact = 0;
+  e.list_up = false;
   for (int64_t col = 0; col < e.hi_col; ++col)
     if (e.h_st[col].active) e.h_gcols[e.nact++] = (int32_t)col;
   // the split-BF16 engine compacts the active columns itself; the others cover [0, hi_col) padded
@@ -2366,7 +2490,7 @@ static int step_launch(sg_ctx* c) {
   SG_CUDA(c, cudaEventRecord(e.ev[1], c->stream));
   const float* Yf = yf ? e.Yf : nullptr;
   const double* Yd = yf ? nullptr : e.Yd;
-  if (!compact_mode(c->mv_mode) && e.nact > 0)  // the compacting engines uploaded the list already
+  if (!e.list_up && e.nact > 0)
     SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, e.nact * 4, cudaMemcpyHostToDevice, c->stream));
   launch_pcg_sigma_dot(e.np, e.nact, e.d_st, e.d_ph, e.winv, e.minv, e.P, Yf, Yd, e.part, e.nblk, e.d_gcols,
                        c->stream);
@@ -3208,7 +3332,7 @@ extern "C" int sg_grm_matmul(sg_ctx* c, const double* V, int64_t k, double* out)
 
 extern "C" int sg_getCrossprodMatAndKin(sg_ctx* c, const float* b, float* out) {
   NEED_OPERATOR(c);
-  DigitsScope digits(c);
+  Fp32Scope scope(c, 1);
   std::vector<double> bd, od(c->nn);
   f2d(b, c->nn, bd);
   SG_TRY(sg_grm_matmul(c, bd.data(), 1, od.data()));
@@ -3259,7 +3383,7 @@ extern "C" int sg_pcg_solve(sg_ctx* c, const double* w, const double* tau, const
 static int solve_f32(sg_ctx* c, const float* w, const float* tau, const float* B, int64_t k, int maxiter,
                      float tol, float* out, int32_t* iters) {
   NEED_OPERATOR(c);
-  DigitsScope digits(c);
+  Fp32Scope scope(c, std::max<int64_t>(k, 1));
   const int64_t n = c->nn;
   if (!all_finite(w, n) || !all_finite(tau, 2)) return set_err(c, SG_ERR_NUMERIC, "W or tau not finite");
   std::vector<double> wd, bd, xd(n * k);
@@ -3325,7 +3449,7 @@ static int trace_common(sg_ctx* c, const float* Sigma_iX, int64_t p, const float
                         bool quant, float* trace, int32_t* nrun_used) {
   NEED_OPERATOR(c);
   if (nrun < 2) return set_err(c, SG_ERR_INVALID, "nrun must be >= 2");
-  DigitsScope digits(c);
+  Fp32Scope scope(c, 2 * nrun);
   SG_TRY(dropin_setup(c, w, tau, 2 * nrun + 4));
   std::vector<double> SX, cv;
   f2d(Sigma_iX, c->nn * p, SX);
@@ -3368,7 +3492,7 @@ int ai_score(sg_ctx* c, const float* Y, const float* X, int64_t p, const float* 
              const float* Sigma_iY, const float* Sigma_iX, const float* cov_in, int nrun, int maxiter,
              float tol, float cutoff, uint64_t seed, bool quant, AIOut* o) {
   NEED_OPERATOR(c);
-  DigitsScope digits(c);
+  Fp32Scope scope(c, 2 * (int64_t)nrun + 3);
   const int64_t n = c->nn;
   SG_TRY(dropin_setup(c, w, tau, 2 * nrun + 8));
   std::vector<double> Yd, Xd, SY, SX, cv;

@@ -433,7 +433,7 @@ __global__ void fp4_gbuild_mm_kernel(const uint8_t* __restrict__ codes, int64_t 
     const int64_t mk = rb * 128 + grp * 8 + row, s0 = (int64_t)ks * kStageK + chunk * 32;
     uint32_t o[4] = {0, 0, 0, 0};
     if (mk < m && s0 < nn) {
-      const uint32_t fc = 2u * (uint32_t)fill[mk];
+      const uint32_t fc = fill ? 2u * (uint32_t)fill[mk] : 0u;
       const uint8_t* src = codes + mk * pitch + s0 / 4;
 #pragma unroll
       for (int w = 0; w < 4; ++w)

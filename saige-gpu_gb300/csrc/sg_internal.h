@@ -82,6 +82,9 @@ void launch_unpack_marker(const uint8_t* packed_row, int64_t nn, const float* lu
 void launch_gemm_nt_f32(const float* A, int64_t lda, const float* B, int64_t ldb, float* C,
                         int64_t ldc, int64_t M, int64_t N, int64_t K, float scale, int mode,
                         cudaStream_t s);
+// Y[:, cols[j]] = K P[:, cols[j]], K (n x n) FP32, n a multiple of 128, columns n apart
+void launch_gemv_multi(const float* K, int64_t n, const float* P, const int32_t* cols, int64_t ncols, float* Y,
+                       cudaStream_t s);
 void launch_gemv_f64(const float* K, int64_t ld, int64_t n, const double* x, double* y,
                      cudaStream_t s);
 
@@ -265,7 +268,8 @@ constexpr int kFp4StageK = 192;   // elements of K per pipeline stage
 constexpr int kFp4PadCols = 64;   // columns a launch may pad its last tile with
 int64_t fp4_matrix_bytes(int64_t rows, int64_t k);  // G in E2M1 stages: rows padded to 256, K to 192
 int64_t fp4_digit_bytes(int64_t cols, int64_t k);   // room for cols columns' digits, whatever the tile
-// G with rows of markers (m x nn) and with rows of samples (nn x m), missing calls at the cohort fill
+// G with rows of markers (m x nn) and with rows of samples (nn x m), missing calls at the cohort fill (fill may
+// be null when there are none)
 void launch_fp4_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int64_t m, int64_t nn, void* Gmm,
                        void* Gsm, cudaStream_t s);
 // columns per tile for a launch over ncols columns (pad ncols to a multiple of it)
@@ -274,6 +278,7 @@ int fp4_tile_cols(int64_t ncols);
 struct Fp4Scratch {
   void *Vq = nullptr, *Tq = nullptr;       // digits of the centred P and of T'
   float *T = nullptr, *U = nullptr;        // cap x mg, cap x np
+  int64_t mg = 0;                          // markers T has room for
   double *part = nullptr, *qsum = nullptr; // cap x nblk block partials each
   float* pmax = nullptr;                   // the same size
   float *mean = nullptr, *descale1 = nullptr, *descale2 = nullptr;  // cap each

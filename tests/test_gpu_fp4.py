@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from oracle import aireml, plink
-from saigegpu import GRM_BF16X3_TC, GRM_FP32_SIMT, MV_FP32_SIMT, MV_SUBSET_EXACT, synth
+from saigegpu import GRM_BF16X3_TC, GRM_FP32_SIMT, MV_BF16X3_TC, MV_FP32_SIMT, MV_SUBSET_EXACT, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -138,3 +138,33 @@ def test_grm_of_a_wide_frequency_range_takes_the_other_builds(gpu_ctx, precision
     ref = aireml.DenseGRM(g).K
     ctx.grm_build(precision)
     assert np.abs(ctx.grm_get() - ref).max() < tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("mode,n,m", [(MV_BF16X3_TC, 500, 900), (MV_BF16X3_TC, 700, 1900), (MV_FP32_SIMT, 129, 300),
+                                      (MV_FP32_SIMT, 1030, 700)])
+def test_drop_ins_on_a_resident_grm(gpu_ctx, mode, n, m):
+    """Two PCG iterations over 1 to 70 columns in the resident-GRM engines: through the genotypes (split BF16, M
+    <= 2.4 N), through K (M above), and through the few-column FP32 kernel.  Split BF16 keeps 16 bits of K and
+    P (2^-17 of each factor, entering twice with coefficients of order one)."""
+    bed, _ = synth.synth_bed(40 + n, n, m, 0.02)
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    grm = aireml.DenseGRM(plink.setgeno(bed, n, m, np.arange(1, n + 1), np.ones(n, bool), 0.01, 0.15))
+    V = np.random.default_rng(n).standard_normal((n, 70)).astype(np.float32)
+    w, tau = np.ones(n, np.float32), np.array([0.5, 0.5], np.float32)
+    ref = aireml.pcg(grm, w, tau, V, 2, 0.0)
+    ctx.grm_build(GRM_BF16X3_TC if mode == MV_BF16X3_TC else GRM_FP32_SIMT)
+    ctx.set_matvec_mode(mode)
+    try:
+        first = None
+        for k in (1, 2, 3, 5, 8, 9, 16, 17, 33, 70):
+            X = ctx.getSigma_X(w, tau, V[:, :k], 2, 0.0)
+            err = np.abs(X - ref[:, :k]).max(0) / np.abs(ref[:, :k]).max(0)
+            assert err.max() < (8 * 2.0 ** -17 if mode == MV_BF16X3_TC else 4 * TOL), (k, err.argmax(), err.max())
+            first = X[:, 0] if first is None else first
+            np.testing.assert_array_equal(X[:, 0], first)  # whatever its neighbours
+        y, want = ctx.getCrossprodMatAndKin(V[:, 0]), grm.K @ V[:, 0].astype(np.float64)
+        assert np.abs(y - want).max() < (4 * 2.0 ** -17 if mode == MV_BF16X3_TC else TOL) * np.abs(want).max()
+    finally:
+        ctx.set_matvec_mode(MV_FP32_SIMT)
