@@ -52,7 +52,6 @@ struct Engine {
   float *Pf = nullptr, *Yf = nullptr;
   ColState* d_st = nullptr;
   PhenoState* d_ph = nullptr;
-  int32_t* d_cols = nullptr;
   std::vector<ColState> h_st;
   std::vector<int64_t> col_req;
   std::vector<PhenoState> h_ph;
@@ -71,12 +70,11 @@ struct Engine {
   int32_t* h_gcols = nullptr;     // pinned: the step's active columns (GRM.V compaction, vector kernels)
   int64_t nact = 0;
   // pinned staging: column states for one scatter launch (h_sst / h_scol, n_sst staged), the
-  // admitted columns and probe tables of an admission round, and slabs holding queued
-  // right-hand sides; all copied up asynchronously
+  // admitted columns and right-hand-side tables of an admission round -- a few hundred bytes that one
+  // thread of each block reads in place, since a copy before a kernel costs more than the read over
+  // the link -- the probe tables, and slabs holding queued right-hand sides
   ColState* h_sst = nullptr;
   int32_t* h_scol = nullptr;
-  ColState* d_sst = nullptr;
-  int32_t* d_scol = nullptr;
   int64_t n_sst = 0;
   std::vector<int32_t> stage_idx;  // column -> its entry in the current staging batch, or -1
   std::vector<int64_t> slab_pending;  // admitted requests whose slabs return once the stream drains
@@ -98,7 +96,7 @@ struct Engine {
   double* d_sx = nullptr;         // probe_dots: Sigma^-1 X block
   double* d_dpart = nullptr;      // probe_dots: block partial sums
   int32_t* d_dcols = nullptr;     // probe_dots: column indices
-  uint8_t* ptab = nullptr;        // probe table of one admission round (stage_cols x 24 B)
+  uint8_t* ptab = nullptr;        // probe table of one admission round (stage_cols x 20 B)
   // K u of each slot's probes, kept between AI-REML iterations (the probes and the slot's sample
   // mask do not change during a fit): kProbeCache vectors per slot, keyed by (seed, run)
   double* pcache = nullptr;
@@ -186,6 +184,10 @@ struct Engine {
   float* smax = nullptr;          // FP16 / E4M3 form: column block maxima, as spart
   float* sscale = nullptr;        //   and the columns' power-of-two scales s1, s2 (2 x cap_cols)
   bool list_up = false;           // the step's active columns are on the device
+  std::vector<int32_t> last_list;  // what d_gcols holds
+  double* pap = nullptr;          // block partials of p'Ap: cap_cols x nblk
+  uint32_t* done = nullptr;       // per column, blocks of the direction kernel that have finished
+  int* h_err = nullptr;           // pinned: the tcgen05 kernels' error flag as of the step's end
   int64_t fp32_cols = 0;          // > 0: a drop-in that returns FP32 runs, with steps of up to so many columns
   Fp4Scratch f4;
   float* sdiag_part[kSetupStreams] = {};  // per-chunk partial sums of a subset's diagonal, per set-up stream
@@ -1465,9 +1467,11 @@ static void engine_free(sg_ctx* c) {
   e.slot_rec.clear();
   e.slot_wait.clear();
   dev_free_t(c, e.X); dev_free_t(c, e.R); dev_free_t(c, e.Z); dev_free_t(c, e.P);
+  dev_free_t(c, e.pap); dev_free_t(c, e.done);
+  e.last_list.clear();
   dev_free_t(c, e.B); dev_free_t(c, e.part); dev_free_t(c, e.winv); dev_free_t(c, e.minv);
   dev_free_t(c, e.Yd); dev_free_t(c, e.Pf); dev_free_t(c, e.Yf); dev_free_t(c, e.d_st);
-  dev_free_t(c, e.d_ph); dev_free_t(c, e.d_cols); dev_free_t(c, e.Pflo);
+  dev_free_t(c, e.d_ph); dev_free_t(c, e.Pflo);
   dev_free(c, e.Pb);
   e.Pb = nullptr;
   dev_free_t(c, e.d_sx); dev_free_t(c, e.d_dpart); dev_free_t(c, e.d_dcols); dev_free_t(c, e.ptab);
@@ -1509,6 +1513,8 @@ static void engine_free(sg_ctx* c) {
   e.pending_release.clear();
   if (e.h_pin) cudaFreeHost(e.h_pin);
   e.h_pin = nullptr;
+  if (e.h_err) cudaFreeHost(e.h_err);
+  e.h_err = nullptr;
   if (e.h_gcols) cudaFreeHost(e.h_gcols);
   e.h_gcols = nullptr;
   for (auto& p : e.d_wstage) dev_free_t(c, p);
@@ -1518,8 +1524,6 @@ static void engine_free(sg_ctx* c) {
     if (*hp) cudaFreeHost(*hp);
     *hp = nullptr;
   }
-  dev_free_t(c, e.d_sst);
-  dev_free_t(c, e.d_scol);
   e.n_sst = 0;
   if (!e.slab_blocks.empty()) cudaStreamSynchronize(c->up);
   for (void* blk : e.slab_blocks) cudaFreeHost(blk);
@@ -1607,12 +1611,14 @@ static int engine_reserve(sg_ctx* c, int64_t max_columns, int64_t max_phenos) {
   SG_TRY(dev_alloc_t(c, &e.Pf, V)); SG_TRY(dev_alloc_t(c, &e.Yf, V));
   SG_TRY(dev_alloc_t(c, &e.B, (size_t)(e.stage_cols * np)));
   SG_TRY(dev_alloc_t(c, &e.part, (size_t)(max_columns * e.nblk * 2)));
-  SG_TRY(dev_alloc_t(c, &e.ptab, (size_t)(e.stage_cols * 36)));  // probe tables | RHS pointers and rows
+  SG_TRY(dev_alloc_t(c, &e.pap, (size_t)(max_columns * e.nblk)));
+  SG_TRY(dev_alloc_t(c, &e.done, (size_t)max_columns));
+  SG_CUDA(c, cudaMemsetAsync(e.done, 0, max_columns * sizeof(uint32_t), c->stream));
+  SG_TRY(dev_alloc_t(c, &e.ptab, (size_t)(e.stage_cols * 20)));
   SG_TRY(dev_alloc_t(c, &e.winv, (size_t)(max_phenos * np)));
   SG_TRY(dev_alloc_t(c, &e.minv, (size_t)(max_phenos * np)));
   SG_TRY(dev_alloc_t(c, &e.d_st, (size_t)max_columns));
   SG_TRY(dev_alloc_t(c, &e.d_ph, (size_t)max_phenos));
-  SG_TRY(dev_alloc_t(c, &e.d_cols, (size_t)max_columns));
   SG_CUDA(c, cudaMemsetAsync(e.Pf, 0, V * 4, c->stream));
   SG_CUDA(c, cudaMemsetAsync(e.P, 0, V * 8, c->stream));
   SG_CUDA(c, cudaMemsetAsync(e.winv, 0, (size_t)(max_phenos * np) * 8, c->stream));
@@ -1629,14 +1635,14 @@ static int engine_reserve(sg_ctx* c, int64_t max_columns, int64_t max_phenos) {
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_pin), max_columns * sizeof(ColState), cudaHostAllocDefault));
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_gcols), (max_columns + kFp4PadCols) * sizeof(int32_t),
                            cudaHostAllocDefault));
+  SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_err), sizeof(int), cudaHostAllocDefault));
+  *e.h_err = 0;
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_sst), max_columns * sizeof(ColState), cudaHostAllocDefault));
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_scol), max_columns * sizeof(int32_t), cudaHostAllocDefault));
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_acols), e.stage_cols * sizeof(int32_t), cudaHostAllocDefault));
   SG_CUDA(c, cudaHostAlloc(reinterpret_cast<void**>(&e.h_ptab), e.stage_cols * 36, cudaHostAllocDefault));
-  SG_TRY(dev_alloc_t(c, &e.d_sst, (size_t)max_columns));
   e.stage_idx.assign(max_columns, -1);
   e.slab_pending.clear();
-  SG_TRY(dev_alloc_t(c, &e.d_scol, (size_t)max_columns));
   for (auto& p : e.d_wstage) SG_TRY(dev_alloc_t(c, &p, (size_t)(2 * np)));
   SG_TRY(dev_alloc_t(c, &e.d_wstage2, (size_t)(2 * np)));
   SG_TRY(dev_alloc_t(c, &e.d_gcols, (size_t)(max_columns + kFp4PadCols)));
@@ -2038,8 +2044,8 @@ extern "C" int sg_engine_submit_chained(sg_ctx* c, int64_t slot, const int64_t* 
   return SG_OK;
 }
 
-// Column-state updates go up in one block: stage (col, state) pairs, then flush_states copies them
-// and scatters them into d_st with one launch.  The pinned staging is reused only after the stream
+// Column-state updates go up in one block: stage (col, state) pairs, then flush_states scatters them
+// into d_st with one launch.  The pinned staging is reused only after the stream
 // has drained past the copy (wait = true, or a later synchronisation on the same stream).
 static void stage_state(Engine& e, int64_t col, const ColState& st) {
   int32_t& at = e.stage_idx[col];
@@ -2059,10 +2065,8 @@ static int flush_states(sg_ctx* c, bool wait) {
   const int64_t n = e.n_sst;
   e.n_sst = 0;
   for (int64_t k = 0; k < n; ++k) e.stage_idx[e.h_scol[k]] = -1;
-  SG_CUDA(c, cudaMemcpyAsync(e.d_sst, e.h_sst, n * sizeof(ColState), cudaMemcpyHostToDevice, c->stream));
-  SG_CUDA(c, cudaMemcpyAsync(e.d_scol, e.h_scol, n * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
   e.io_h2d += (uint64_t)(n * (sizeof(ColState) + sizeof(int32_t)));
-  launch_scatter_states(e.d_sst, e.d_scol, n, e.d_st, e.Pf, e.np, c->stream);
+  launch_scatter_states(e.h_sst, e.h_scol, n, e.d_st, e.Pf, e.np, c->stream);
   SG_LAUNCHED(c, 1);
   return wait ? sync(c) : SG_OK;
 }
@@ -2242,9 +2246,8 @@ static int engine_admit(sg_ctx* c) {
       unsigned char* hb = e.h_ptab + e.stage_cols * 24;
       std::memcpy(hb, rsrc.data(), kr * sizeof(void*));
       std::memcpy(hb + kr * sizeof(void*), rsel.data(), kr * 4);
-      unsigned char* db = reinterpret_cast<unsigned char*>(e.ptab) + e.stage_cols * 24;
-      SG_CUDA(c, h2d(c, db, hb, kr * (sizeof(void*) + 4), c->stream));
-      launch_gather_rhs(reinterpret_cast<const double* const*>(db), reinterpret_cast<const int32_t*>(db + kr * sizeof(void*)),
+      e.io_h2d += kr * (sizeof(void*) + 4);
+      launch_gather_rhs(reinterpret_cast<const double* const*>(hb), reinterpret_cast<const int32_t*>(hb + kr * sizeof(void*)),
                         (int64_t)kr, c->nn, e.np, e.B, c->stream);
       SG_LAUNCHED(c, 1);
     }
@@ -2258,6 +2261,7 @@ static int engine_admit(sg_ctx* c) {
       std::memcpy(h_seeds, pseeds.data(), kp * 8);
       std::memcpy(h_runs, pruns.data(), kp * 8);
       std::memcpy(h_sel, psel.data(), kp * 4);
+      // thousands of blocks read this one: it goes up
       SG_CUDA(c, h2d(c, e.ptab, e.h_ptab, kp * 20, c->stream));
       uint64_t* d_seeds = reinterpret_cast<uint64_t*>(e.ptab);
       int64_t* d_runs = reinterpret_cast<int64_t*>(d_seeds + kp);
@@ -2266,8 +2270,8 @@ static int engine_admit(sg_ctx* c) {
       c->launches += 1;
     }
     std::memcpy(e.h_acols, cols.data(), cols.size() * 4);
-    SG_CUDA(c, h2d(c, e.d_cols, e.h_acols, cols.size() * 4, c->stream));
-    launch_pcg_init(e.np, e.cap_cols, e.d_cols, (int64_t)cols.size(), e.d_st, e.d_ph, e.minv, e.B,
+    e.io_h2d += cols.size() * 4;
+    launch_pcg_init(e.np, e.cap_cols, e.h_acols, (int64_t)cols.size(), e.d_st, e.d_ph, e.minv, e.B,
                     e.X, e.R, e.Z, e.P, e.Pf, e.part, e.nblk, c->stream);
     SG_LAUNCHED(c, 2);
     // for the FP64 plain engine the product columns read P: stage b there too
@@ -2284,6 +2288,18 @@ static int engine_admit(sg_ctx* c) {
     if ((int64_t)cols.size() < e.stage_cols) break;
   }
   return flush_states(c, false);  // releases with no admission round after them
+}
+
+// The step's active columns on the device, padded with -1 to npad; not copied again while they are those of
+// the last step.
+static int upload_list(sg_ctx* c, int64_t npad) {
+  Engine& e = c->eng;
+  for (int64_t j = e.nact; j < npad; ++j) e.h_gcols[j] = -1;
+  e.list_up = true;
+  if ((int64_t)e.last_list.size() == npad && std::memcmp(e.last_list.data(), e.h_gcols, npad * 4) == 0) return SG_OK;
+  e.last_list.assign(e.h_gcols, e.h_gcols + npad);
+  SG_CUDA(c, h2d(c, e.d_gcols, e.h_gcols, npad * 4, c->stream));
+  return SG_OK;
 }
 
 static int loco_correct(sg_ctx* c, int64_t ncols, bool yf);
@@ -2309,9 +2325,7 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
     const bool subset = exact_mode(c->mv_mode);
     const int ct = form == Fp32Form::kGemv ? 1 : fp4_tile_cols(nact);
     const int64_t npad = round_up(nact, ct);
-    for (int64_t j = nact; j < npad; ++j) e.h_gcols[j] = -1;
-    SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, npad * 4, cudaMemcpyHostToDevice, c->stream));
-    e.list_up = true;
+    SG_TRY(upload_list(c, npad));
     int nl = 1;
     if (form == Fp32Form::kGemv) {
       launch_gemv_multi(c->d_K, e.np, e.Pf, e.d_gcols, nact, e.Yf, c->stream);
@@ -2349,9 +2363,7 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
       return SG_OK;
     }
     const int64_t npad = tc_grmv_padded_cols(round_up(nact, 16), e.cap_cols, e.np, kTilesSplitBF16, c->num_sms);
-    for (int64_t j = nact; j < npad; ++j) e.h_gcols[j] = -1;
-    SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, npad * 4, cudaMemcpyHostToDevice, c->stream));
-    e.list_up = true;
+    SG_TRY(upload_list(c, npad));
     uint16_t* ph = static_cast<uint16_t*>(e.Pb);
     launch_split_bf16_gather(e.Pf, e.np, e.d_gcols, npad, ph, ph + half, c->stream);
     c->launches += 1;
@@ -2372,9 +2384,7 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
     }
     const int64_t np = e.np, mg = c->mg;
     const int64_t npad = tc_grmv_padded_cols(round_up(nact, 32), e.cap_cols, np, kTilesSplitB, c->num_sms);
-    for (int64_t j = nact; j < npad; ++j) e.h_gcols[j] = -1;
-    SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, npad * 4, cudaMemcpyHostToDevice, c->stream));
-    e.list_up = true;
+    SG_TRY(upload_list(c, npad));
     const size_t cap = (size_t)e.cap_cols;
     if (!e.Vb) SG_TRY(dev_alloc(c, &e.Vb, cap * np * 4));
     if (!e.Tm) SG_TRY(dev_alloc_t(c, &e.Tm, cap * mg));
@@ -2490,16 +2500,14 @@ static int step_launch(sg_ctx* c) {
   SG_CUDA(c, cudaEventRecord(e.ev[1], c->stream));
   const float* Yf = yf ? e.Yf : nullptr;
   const double* Yd = yf ? nullptr : e.Yd;
-  if (!e.list_up && e.nact > 0)
-    SG_CUDA(c, cudaMemcpyAsync(e.d_gcols, e.h_gcols, e.nact * 4, cudaMemcpyHostToDevice, c->stream));
-  launch_pcg_sigma_dot(e.np, e.nact, e.d_st, e.d_ph, e.winv, e.minv, e.P, Yf, Yd, e.part, e.nblk, e.d_gcols,
+  if (!e.list_up) SG_TRY(upload_list(c, e.nact));
+  launch_pcg_sigma_dot(e.np, e.nact, e.d_st, e.d_ph, e.winv, e.minv, e.P, Yf, Yd, e.pap, e.nblk, e.d_gcols,
                        c->stream);
-  launch_pcg_alpha(e.nact, e.d_st, e.part, e.nblk, e.d_gcols, c->stream);
-  launch_pcg_update(e.np, e.nact, e.d_st, e.d_ph, e.winv, e.minv, e.X, e.R, e.Z, e.P, Yf, Yd,
+  launch_pcg_update(e.np, e.nact, e.d_st, e.d_ph, e.winv, e.minv, e.X, e.R, e.Z, e.P, Yf, Yd, e.pap,
                     e.part, e.nblk, e.d_gcols, c->stream);
-  launch_pcg_beta(e.nact, e.d_st, e.part, e.nblk, e.d_gcols, c->stream);
-  launch_pcg_dir(e.np, e.nact, e.d_st, e.Z, e.P, e.Pf, e.d_gcols, c->stream);
-  SG_LAUNCHED(c, 5);
+  const int* err = tc_mode(c->mv_mode) ? tc_error_address() : nullptr;
+  launch_pcg_dir(e.np, e.nact, e.d_st, e.Z, e.P, e.Pf, e.part, e.nblk, e.done, e.d_gcols, err, e.h_err, c->stream);
+  SG_LAUNCHED(c, 3);
   SG_CUDA(c, cudaEventRecord(e.ev[2], c->stream));
   SG_CUDA(c, d2h(c, e.h_pin, e.d_st, e.hi_col * sizeof(ColState), c->stream));
   e.inflight = true;
@@ -2516,7 +2524,8 @@ static int step_finish(sg_ctx* c, int64_t* n_finished) {
   e.inflight = false;
   SG_TRY(sync(c));
   const auto th0 = std::chrono::steady_clock::now();
-  if (tc_mode(c->mv_mode)) {
+  if (tc_mode(c->mv_mode) && *e.h_err != 0) {  // a bounded wait gave up: read and clear the device's flag
+    *e.h_err = 0;
     const cudaError_t err = tc_check_error(c->stream);
     if (err != cudaSuccess) return set_err(c, SG_ERR_CUDA, "tcgen05 GRM.V: %s", cudaGetErrorString(err));
   }
@@ -2600,41 +2609,6 @@ static int engine_step(sg_ctx* c, int64_t* n_finished) {
   return step_finish(c, n_finished);
 }
 
-// Columns admitted with r'r <= tol retire without a step (iter = 0, x = 0).
-static int engine_retire_immediate(sg_ctx* c, int64_t* n_finished) {
-  Engine& e = c->eng;
-  if (e.hi_col == 0) return SG_OK;
-  SG_CUDA(c, d2h(c, e.h_st.data(), e.d_st, e.hi_col * sizeof(ColState), c->stream));
-  SG_TRY(sync(c));
-  for (int64_t col = 0; col < e.hi_col; ++col) {
-    const int64_t id = e.col_req[col];
-    if (id < 0) continue;
-    ColState& s = e.h_st[col];
-    if (s.kind != 0 || s.active || !s.just_done) continue;
-    auto it = e.reqs.find(id);
-    if (it != e.reqs.end()) {
-      it->second.iters = 0;
-      it->second.state = 2;
-      it->second.col = e.hold ? col : -1;  // X[col] was zeroed at admission
-      if (!e.hold) it->second.x.assign(c->nn, 0.0);
-      e.finished.push_back(id);
-    }
-    e.n_active -= 1;
-    e.retired += 1;
-    *n_finished += 1;
-    if (e.hold && it != e.reqs.end()) {
-      s.kind = -2;
-      s.just_done = 0;
-      stage_state(e, col, s);
-    } else {
-      SG_TRY(release_col(c, col));
-    }
-  }
-  while (e.hi_col > 0 && e.col_req[e.hi_col - 1] == -1) --e.hi_col;
-  SG_TRY(flush_states(c, false));
-  return sync(c);
-}
-
 extern "C" int sg_engine_run(sg_ctx* c, int64_t max_steps, int64_t* n_finished) {
   NEED_OPERATOR(c);
   Engine& e = c->eng;
@@ -2649,8 +2623,8 @@ extern "C" int sg_engine_run(sg_ctx* c, int64_t max_steps, int64_t* n_finished) 
   }
   for (int64_t s = 0; s < max_steps; ++s) {
     SG_TRY(engine_admit(c));
-    SG_TRY(engine_retire_immediate(c, &fin));
-    if (fin > 0) break;
+    // columns that converged at init (iter = 0, x = 0) retire when this step finishes: reading the fresh
+    // states back first would cost every call a round trip
     if (e.n_active == 0) {
       if (!e.queue.empty())
         return set_err(c, SG_ERR_STATE,

@@ -65,8 +65,11 @@ __global__ void pcg_init_kernel(int64_t np, const int32_t* __restrict__ cols,
                                 const double* __restrict__ B, double* X, double* R, double* Z,
                                 double* P, float* Pf, double* part, int64_t nblk) {
   __shared__ double sh[kThreads / 32];
+  __shared__ int s_col;
   const int sel = blockIdx.y;
-  const int64_t c = cols[sel];
+  if (threadIdx.x == 0) s_col = cols[sel];  // pinned host memory
+  __syncthreads();
+  const int64_t c = s_col;
   const ColState s = st[c];
   const double* mv = minv + (int64_t)s.pheno * np;
   const double* b = B + (int64_t)sel * np;
@@ -116,8 +119,6 @@ __global__ void pcg_init_finalize_kernel(const int32_t* __restrict__ cols, int64
   }
   s.iter = 0;
   s.just_done = 0;
-  s.alpha = 0.0;
-  s.beta = 0.0;
   if (s.kind == 0) {
     s.rz = zr;
     s.r2 = rr;
@@ -151,15 +152,12 @@ __global__ void pcg_sigma_dot_kernel(int64_t np, const ColState* __restrict__ st
                                      const PhenoState* __restrict__ ph,
                                      const double* __restrict__ winv, const double* __restrict__ minv,
                                      const double* __restrict__ P, const float* __restrict__ Yf,
-                                     const double* __restrict__ Yd, double* part, int64_t nblk,
+                                     const double* __restrict__ Yd, double* pap, int64_t nblk,
                                      const int32_t* __restrict__ cols) {
   __shared__ double sh[kThreads / 32];
-  const int64_t c = cols ? cols[blockIdx.y] : blockIdx.y;
+  const int64_t c = cols[blockIdx.y];
   const ColState s = st[c];
-  if (s.kind != 0 || !s.active) {
-    if (threadIdx.x == 0) part[(c * nblk + blockIdx.x) * 2] = 0.0;
-    return;
-  }
+  if (s.kind != 0 || !s.active) return;
   const PhenoState g = ph[s.pheno];
   const double* wv = winv + (int64_t)s.pheno * np;
   const double* mv = minv + (int64_t)s.pheno * np;
@@ -175,59 +173,34 @@ __global__ void pcg_sigma_dot_kernel(int64_t np, const ColState* __restrict__ st
     acc += p.y * ap_value(g.tau0, g.tau1, w.y, m.y, p.y, y.y);
   }
   acc = block_sum(acc, sh);
-  if (threadIdx.x == 0) part[(c * nblk + blockIdx.x) * 2] = acc;
+  if (threadIdx.x == 0) pap[c * nblk + blockIdx.x] = acc;
 }
 
 void launch_pcg_sigma_dot(int64_t np, int64_t ncols, ColState* st, const PhenoState* ph,
                           const double* winv, const double* minv, const double* P,
-                          const float* Yf, const double* Yd, double* part, int64_t nblk,
+                          const float* Yf, const double* Yd, double* pap, int64_t nblk,
                           const int32_t* cols, cudaStream_t s) {
   if (ncols == 0) return;
   dim3 grid((unsigned)nblk, (unsigned)ncols);
-  pcg_sigma_dot_kernel<<<grid, kThreads, 0, s>>>(np, st, ph, winv, minv, P, Yf, Yd, part, nblk, cols);
+  pcg_sigma_dot_kernel<<<grid, kThreads, 0, s>>>(np, st, ph, winv, minv, P, Yf, Yd, pap, nblk, cols);
 }
 
-__global__ void pcg_alpha_kernel(int64_t ncols, ColState* st, const double* __restrict__ part,
-                                 int64_t nblk, const int32_t* __restrict__ cols) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= ncols) return;
-  const int64_t c = cols ? cols[j] : j;
-  ColState s = st[c];
-  if (s.kind != 0 || !s.active) {
-    s.alpha = 0.0;
-  } else {
-    double pap = 0.0;
-    for (int64_t b = 0; b < nblk; ++b) pap += part[(c * nblk + b) * 2];
-    s.alpha = s.rz / pap;
-  }
-  st[c].alpha = s.alpha;
-}
-
-void launch_pcg_alpha(int64_t ncols, ColState* st, const double* part, int64_t nblk,
-                      const int32_t* cols, cudaStream_t s) {
-  if (ncols == 0) return;
-  pcg_alpha_kernel<<<(unsigned)((ncols + 127) / 128), 128, 0, s>>>(ncols, st, part, nblk, cols);
-}
-
-// x += a p; r -= a Ap; z = minv r; partial z'r, r'r.  Product columns copy K b into X.
+// x += a p; r -= a Ap; z = minv r; partial z'r, r'r.  Product columns copy K b into X.  Every block of a
+// column adds the partials of p'Ap itself, in block order, so no kernel stands between the two (a
+// separate one took 4.7 us of every step: a serial sum behind a launch).
 __global__ void pcg_update_kernel(int64_t np, const ColState* __restrict__ st,
                                   const PhenoState* __restrict__ ph, const double* __restrict__ winv,
                                   const double* __restrict__ minv, double* X, double* R, double* Z,
                                   const double* __restrict__ P, const float* __restrict__ Yf,
-                                  const double* __restrict__ Yd, double* part, int64_t nblk,
-                                  const int32_t* __restrict__ cols) {
+                                  const double* __restrict__ Yd, const double* __restrict__ pap, double* part,
+                                  int64_t nblk, const int32_t* __restrict__ cols) {
   __shared__ double sh[kThreads / 32];
-  const int64_t c = cols ? cols[blockIdx.y] : blockIdx.y;
+  __shared__ double s_alpha;
+  const int64_t c = cols[blockIdx.y];
   const ColState s = st[c];
   const int64_t base = c * np;
   const int64_t i0 = (int64_t)blockIdx.x * kChunk;
-  if (!s.active) {
-    if (threadIdx.x == 0) {
-      part[(c * nblk + blockIdx.x) * 2 + 0] = 0.0;
-      part[(c * nblk + blockIdx.x) * 2 + 1] = 0.0;
-    }
-    return;
-  }
+  if (!s.active) return;
   const double* mv = minv + (int64_t)s.pheno * np;
   if (s.kind == 1) {
 #pragma unroll
@@ -241,7 +214,13 @@ __global__ void pcg_update_kernel(int64_t np, const ColState* __restrict__ st,
   }
   const PhenoState g = ph[s.pheno];
   const double* wv = winv + (int64_t)s.pheno * np;
-  const double a = s.alpha;
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int64_t b = 0; b < nblk; ++b) t += pap[c * nblk + b];
+    s_alpha = s.rz / t;
+  }
+  __syncthreads();
+  const double a = s_alpha;
   double zr = 0.0, rr = 0.0;
 #pragma unroll
   for (int it = 0; it < kVecIters; ++it) {
@@ -271,60 +250,54 @@ __global__ void pcg_update_kernel(int64_t np, const ColState* __restrict__ st,
 
 void launch_pcg_update(int64_t np, int64_t ncols, ColState* st, const PhenoState* ph,
                        const double* winv, const double* minv, double* X, double* R, double* Z,
-                       const double* P, const float* Yf, const double* Yd, double* part,
+                       const double* P, const float* Yf, const double* Yd, const double* pap, double* part,
                        int64_t nblk, const int32_t* cols, cudaStream_t s) {
   if (ncols == 0) return;
   dim3 grid((unsigned)nblk, (unsigned)ncols);
-  pcg_update_kernel<<<grid, kThreads, 0, s>>>(np, st, ph, winv, minv, X, R, Z, P, Yf, Yd, part, nblk, cols);
+  pcg_update_kernel<<<grid, kThreads, 0, s>>>(np, st, ph, winv, minv, X, R, Z, P, Yf, Yd, pap, part, nblk, cols);
 }
 
-// beta, iteration count and the stopping rule (sum r^2 <= tol or iter == maxiter)
-__global__ void pcg_beta_kernel(int64_t ncols, ColState* st, const double* __restrict__ part,
-                                int64_t nblk, const int32_t* __restrict__ cols) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= ncols) return;
-  const int64_t c = cols ? cols[j] : j;
+// beta, the iteration count and the stopping rule (sum r^2 <= tol or iter == maxiter), then p = z + beta p for
+// columns still iterating with an FP32 copy for the next GRM product; columns that have just finished get
+// a zero FP32 direction.  Every block of a column adds the partials of z'r and r'r itself, in block order; the
+// last of them to finish writes the column's new state (``done`` counts them and returns to zero), since
+// the others read the old one.
+__global__ void pcg_dir_kernel(int64_t np, ColState* __restrict__ st, const double* __restrict__ Z, double* P,
+                               float* Pf, const double* __restrict__ part, int64_t nblk, uint32_t* __restrict__ done,
+                               const int32_t* __restrict__ cols, const int* __restrict__ err,
+                               int* __restrict__ err_out) {
+  __shared__ double s_zr, s_rr;
+  const int64_t c = cols[blockIdx.y];
   ColState s = st[c];
-  s.just_done = 0;
-  if (s.active) {
-    if (s.kind == 1) {
-      s.active = 0;
-      s.just_done = 1;
-      s.iter = 1;
-    } else {
-      double zr = 0.0, rr = 0.0;
-      for (int64_t b = 0; b < nblk; ++b) {
-        zr += part[(c * nblk + b) * 2 + 0];
-        rr += part[(c * nblk + b) * 2 + 1];
-      }
-      s.beta = zr / s.rz;
-      s.rz = zr;
-      s.r2 = rr;
-      s.iter += 1;
-      if (!(rr > s.tol && s.iter < s.maxiter)) {
-        s.active = 0;
-        s.just_done = 1;
-      }
-    }
-  }
-  st[c] = s;
-}
-
-void launch_pcg_beta(int64_t ncols, ColState* st, const double* part, int64_t nblk,
-                     const int32_t* cols, cudaStream_t s) {
-  if (ncols == 0) return;
-  pcg_beta_kernel<<<(unsigned)((ncols + 127) / 128), 128, 0, s>>>(ncols, st, part, nblk, cols);
-}
-
-// p = z + beta p for columns still iterating; FP32 copy for the next GRM product.
-__global__ void pcg_dir_kernel(int64_t np, const ColState* __restrict__ st, const double* __restrict__ Z,
-                               double* P, float* Pf, const int32_t* __restrict__ cols) {
-  const int64_t c = cols ? cols[blockIdx.y] : blockIdx.y;
-  const ColState s = st[c];
   const int64_t base = c * np;
   const int64_t i0 = (int64_t)blockIdx.x * kChunk;
-  if (s.active && s.kind == 0) {
-    const double b = s.beta;
+  s.just_done = 0;
+  double b = 0.0;
+  if (s.active && s.kind == 1) {
+    s.active = 0;
+    s.just_done = 1;
+    s.iter = 1;
+  } else if (s.active) {
+    if (threadIdx.x == 0) {
+      double zr = 0.0, rr = 0.0;
+      for (int64_t q = 0; q < nblk; ++q) {
+        zr += part[(c * nblk + q) * 2 + 0];
+        rr += part[(c * nblk + q) * 2 + 1];
+      }
+      s_zr = zr;
+      s_rr = rr;
+    }
+    __syncthreads();
+    b = s_zr / s.rz;
+    s.rz = s_zr;
+    s.r2 = s_rr;
+    s.iter += 1;
+    if (!(s.r2 > s.tol && s.iter < s.maxiter)) {
+      s.active = 0;
+      s.just_done = 1;
+    }
+  }
+  if (s.active) {
 #pragma unroll
     for (int it = 0; it < kVecIters; ++it) {
       const int64_t i = i0 + 2 * (it * kThreads + threadIdx.x);
@@ -342,13 +315,23 @@ __global__ void pcg_dir_kernel(int64_t np, const ColState* __restrict__ st, cons
       st2f(Pf + base + i, 0.0f, 0.0f);
     }
   }
+  __syncthreads();  // every thread of the block has read the old state
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicInc(done + c, (unsigned)nblk - 1u) == (unsigned)nblk - 1u) {
+      __threadfence();
+      st[c] = s;
+    }
+    if (err && blockIdx.x == 0 && blockIdx.y == 0) *err_out = *err;  // rides the states' read-back
+  }
 }
 
 void launch_pcg_dir(int64_t np, int64_t ncols, ColState* st, const double* Z, double* P, float* Pf,
-                    const int32_t* cols, cudaStream_t s) {
+                    const double* part, int64_t nblk, uint32_t* done, const int32_t* cols, const int* err, int* err_out,
+                    cudaStream_t s) {
   if (ncols == 0) return;
-  dim3 grid((unsigned)pcg_nblk(np), (unsigned)ncols);
-  pcg_dir_kernel<<<grid, kThreads, 0, s>>>(np, st, Z, P, Pf, cols);
+  dim3 grid((unsigned)nblk, (unsigned)ncols);
+  pcg_dir_kernel<<<grid, kThreads, 0, s>>>(np, st, Z, P, Pf, part, nblk, done, cols, err, err_out);
 }
 
 // Rademacher probes of the counter hash (oracle/probes.py): B[j][i] = +-1 for i < nn, 0 after.
@@ -484,17 +467,23 @@ void launch_slot_weights(int64_t np, int64_t nn, const double* w, const uint8_t*
                                                                    diag_one, winv, minv);
 }
 
-// d_st[cols[k]] = src[k]: column states staged by the host in one block; a column set free
+// d_st[cols[k]] = src[k]: column states staged by the host in pinned memory; a column set free
 // (kind -1) also gets a zero FP32 direction, so padding columns of a GRM.V pass contribute nothing.
 // One block per staged column.
 __global__ void scatter_states_kernel(const ColState* __restrict__ src, const int32_t* __restrict__ cols,
                                       int64_t n, ColState* __restrict__ dst, float* __restrict__ Pf, int64_t np) {
+  __shared__ int s_col, s_kind;
   const int64_t k = blockIdx.x;
   if (k >= n) return;
-  const ColState st = src[k];
-  const int64_t c = cols[k];
-  if (threadIdx.x == 0) dst[c] = st;
-  if (Pf && st.kind == -1)
+  if (threadIdx.x == 0) {
+    const ColState st = src[k];
+    s_col = cols[k];
+    s_kind = st.kind;
+    dst[s_col] = st;
+  }
+  __syncthreads();
+  const int64_t c = s_col;
+  if (Pf && s_kind == -1)
     for (int64_t i = threadIdx.x; i < np; i += blockDim.x) Pf[c * np + i] = 0.0f;
 }
 
@@ -504,14 +493,21 @@ void launch_scatter_states(const ColState* src, const int32_t* cols, int64_t n, 
   scatter_states_kernel<<<(unsigned)n, 256, 0, s>>>(src, cols, n, dst, Pf, np);
 }
 
-// Right-hand sides of an admission round: column sel[k] of B (np rows) = the nn values at host
-// address src[k] (pinned and mapped), zero past nn.  One block per column.
+// Right-hand sides of an admission round: column sel[k] of B (np rows) = the nn values at device address
+// src[k], zero past nn.  One block per column; the two tables are pinned host memory.
 __global__ void gather_rhs_kernel(const double* const* __restrict__ src, const int32_t* __restrict__ sel,
                                   int64_t n, int64_t nn, int64_t np, double* __restrict__ B) {
+  __shared__ const double* s_x;
+  __shared__ int s_sel;
   const int64_t k = blockIdx.x;
   if (k >= n) return;
-  const double* x = src[k];
-  double* b = B + (int64_t)sel[k] * np;
+  if (threadIdx.x == 0) {
+    s_x = src[k];
+    s_sel = sel[k];
+  }
+  __syncthreads();
+  const double* x = s_x;
+  double* b = B + (int64_t)s_sel * np;
   for (int64_t i = threadIdx.x; i < np; i += blockDim.x) b[i] = i < nn ? x[i] : 0.0;
 }
 

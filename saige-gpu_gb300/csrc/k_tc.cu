@@ -1373,6 +1373,8 @@ cudaError_t tc_check_error(cudaStream_t s) { return check_error_flag(s); }
 
 PFN_cuTensorMapEncodeTiled_v12000 tc::tc_encode_fn() { return encode_fn(); }
 
+int* tc_error_address() { return tc::tc_error_flag(); }
+
 int* tc::tc_error_flag() {
   void* p = nullptr;
   return cudaGetSymbolAddress(&p, g_tc_error) == cudaSuccess ? static_cast<int*>(p) : nullptr;

@@ -111,6 +111,8 @@ void launch_split_bf16_gather(const float* x, int64_t np, const int32_t* cols, i
                               void* lo, cudaStream_t s);
 // x (+ x2 when not null) = hi + lo, both BF16 (round to nearest even), lo = bf16(x - hi)
 void launch_split_bf16(const float* x, const float* x2, void* hi, void* lo, int64_t n, cudaStream_t s);
+// The flag's device address (nullptr on failure)
+int* tc_error_address();
 // Synchronises s, then reads and clears the flag the tcgen05 kernels set when a bounded wait ran
 // out (cudaErrorLaunchTimeout in that case).
 cudaError_t tc_check_error(cudaStream_t s);
@@ -165,7 +167,6 @@ struct ColState {
   double tol;
   double rz;        // r'z of the current iterate
   double r2;        // r'r
-  double alpha, beta;
 };
 struct PhenoState {
   double tau0, tau1;
@@ -174,31 +175,29 @@ void launch_pcg_init(int64_t np, int64_t ncols, const int32_t* cols, int64_t nco
                      ColState* st, const PhenoState* ph, const double* minv, const double* B,
                      double* X, double* R, double* Z, double* P, float* Pf, double* part,
                      int64_t nblk, cudaStream_t s);
-// The step kernels act on ncols columns: cols[0..ncols) when cols is not null (the active list),
-// else columns 0..ncols-1.
+// The step kernels act on the ncols columns cols[0..ncols): three launches, the scalars between them summed from
+// the block partials by each block in the same order.  pap: nblk per column; part: 2 nblk per column; done: a
+// zeroed counter per column; err (may be null) is copied to err_out.
 void launch_pcg_sigma_dot(int64_t np, int64_t ncols, ColState* st, const PhenoState* ph,
                           const double* winv, const double* minv, const double* P,
-                          const float* Yf, const double* Yd, double* part, int64_t nblk,
+                          const float* Yf, const double* Yd, double* pap, int64_t nblk,
                           const int32_t* cols, cudaStream_t s);
-void launch_pcg_alpha(int64_t ncols, ColState* st, const double* part, int64_t nblk,
-                      const int32_t* cols, cudaStream_t s);
 void launch_pcg_update(int64_t np, int64_t ncols, ColState* st, const PhenoState* ph,
                        const double* winv, const double* minv, double* X, double* R, double* Z,
-                       const double* P, const float* Yf, const double* Yd, double* part,
+                       const double* P, const float* Yf, const double* Yd, const double* pap, double* part,
                        int64_t nblk, const int32_t* cols, cudaStream_t s);
-void launch_pcg_beta(int64_t ncols, ColState* st, const double* part, int64_t nblk,
-                     const int32_t* cols, cudaStream_t s);
-void launch_pcg_dir(int64_t np, int64_t ncols, ColState* st, const double* Z, double* P,
-                    float* Pf, const int32_t* cols, cudaStream_t s);
+void launch_pcg_dir(int64_t np, int64_t ncols, ColState* st, const double* Z, double* P, float* Pf,
+                    const double* part, int64_t nblk, uint32_t* done, const int32_t* cols, const int* err, int* err_out,
+                    cudaStream_t s);
 void launch_probe_fill(int64_t np, int64_t nn, uint64_t seed, int64_t run0, int64_t k,
                        double* B, cudaStream_t s);
 void launch_probe_fill_multi(int64_t np, int64_t nn, const uint64_t* seeds, const int64_t* runs,
                              const int32_t* sel, int64_t k, double* B, cudaStream_t s);
 void launch_f64_to_f32(const double* a, float* b, int64_t n, cudaStream_t s);
-// d_st[cols[k]] = src[k] for k < n; with Pf, columns set free (kind -1) also get P = 0
+// d_st[cols[k]] = src[k] for k < n (src, cols: pinned host memory); with Pf, columns set free (kind -1) also get P = 0
 void launch_scatter_states(const ColState* src, const int32_t* cols, int64_t n, ColState* dst, float* Pf,
                            int64_t np, cudaStream_t s);
-// B[:, sel[k]] = the nn doubles at mapped pinned host address src[k], zero-padded to np
+// B[:, sel[k]] = the nn doubles at device address src[k], zero-padded to np; src and sel are pinned host memory
 void launch_gather_rhs(const double* const* src, const int32_t* sel, int64_t n, int64_t nn, int64_t np, double* B,
                        cudaStream_t s);
 // 1/W and 1/diag(Sigma) of a phenotype slot from W on the device (mask: nullptr = every sample)
