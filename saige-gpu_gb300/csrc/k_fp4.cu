@@ -250,7 +250,7 @@ fp4_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
   if (warp == kProducerWarp4) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int64_t ra = (int64_t)row_block * stages, rb = (int64_t)bt * stages * 2 + crank;
       int issued = 0;
       for (int kb = 0; kb < stages; ++kb) {
@@ -269,7 +269,7 @@ fp4_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
           mbar_wait_teardown(&full[kb % S], (uint32_t)(kb / S) & 1u);
     }
   } else if (warp == kMmaWarp4) {
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       const uint32_t empty_peer = cluster_addr(empty, 1), accf_peer = cluster_addr(acc_full, 1);
       int kb = 0;
       bool go = true;

@@ -286,7 +286,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   const int nchunks = (num_kb + drain_kb - 1) / drain_kb;
 
   if (warp == kProducerWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---------------- TMA producer (each CTA of a pair loads its own operand rows)
       const int32_t ya = row_block * kTileM, yb = tc.bn * BN + (int32_t)crank * kBRows;
       for (int kb = 0; kb < num_kb; ++kb) {
@@ -343,7 +343,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
       }
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       // ---------------- MMA issuer: chunk ch of drain_kb stages goes to accumulator ch % 2, which is
       // reused once the drain warps have read it (two chunks earlier)
       uint32_t empty_peer = 0, accf_peer = 0;

@@ -52,17 +52,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // Bounded wait: returns false (and records ``code`` at ``err``) when the budget runs out
-// or another thread of this kernel already gave up.
+// or another thread of this kernel already gave up.  The global timer is read only after 64 failed
+// tries: a read takes longer than most waits of a pipeline in flow.
 __device__ __forceinline__ bool mbar_wait_budget(uint64_t* bar, uint32_t parity, int code,
                                                  volatile int* abort_flag, unsigned long long budget_ns,
                                                  int* err) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = gtimer();
+  unsigned long long t0 = 0;
   for (uint32_t it = 1;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 255u) == 0u) {
+    if ((it & 63u) == 0u) {
       if (*abort_flag) return false;
-      if (gtimer() - t0 > budget_ns) {
+      const unsigned long long t = gtimer();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > budget_ns) {
         *abort_flag = 1;
         atomicCAS(err, 0, code);
         return false;
@@ -81,14 +83,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int co
 __device__ __forceinline__ bool mbar_wait_sleep(uint64_t* bar, uint32_t parity, int code,
                                                 volatile int* abort_flag, int* err) {
   if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = gtimer();
+  unsigned long long t0 = 0;
   unsigned ns = 32;
-  for (;;) {
+  for (uint32_t it = 1;; ++it) {
     __nanosleep(ns);
     if (mbar_try_wait(bar, parity)) return true;
     if (ns < 256) ns <<= 1;
+    if ((it & 15u) != 0u) continue;
     if (*abort_flag) return false;
-    if (gtimer() - t0 > kWaitBudgetNs) {
+    const unsigned long long t = gtimer();
+    if (t0 == 0) t0 = t;
+    if (t - t0 > kWaitBudgetNs) {
       *abort_flag = 1;
       atomicCAS(err, 0, code);
       return false;
@@ -113,6 +118,15 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
+// One lane of a converged warp, by elect.sync: the compiler then keeps the operands of what that lane issues
+// (tcgen05.mma, TMA, commits) in uniform registers.  Behind a test of the lane number the same MMA loop took 45 clocks an
+// instruction, behind this 17 (128 x 32 x 16 BF16, its operands' own rate).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.b32 %0, 1, 0, q;\n\t}" : "=r"(e));
+  return e != 0;
+}
+
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -130,9 +144,11 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
   return r;
 }
 
-// Arrive once on an mbarrier given by its cluster address (this CTA's or the peer's).
+// Arrive once on an mbarrier given by its cluster address (this CTA's or the peer's), with the default release
+// at CTA scope: what these arrivals publish is in TMEM, ordered by the tcgen05 waits and fences before
+// them.  (A release at cluster scope took 1,000-1,300 clocks of the arriving warp.)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
 }
 
 // CTA-pair load: the box lands in this CTA's shared memory and completes its transaction bytes on
