@@ -271,6 +271,10 @@ struct sg_ctx {
   void* d_G = nullptr;   // genotype matrix: BF16 (form 0) or FP16 then E4M3 (form 1), both layouts each
   int g_form = 0;
   int64_t mg = 0;
+  // the same values in two bits for the products of few columns, built at the first of them
+  void* d_Gp = nullptr;
+  bool gp_refused = false;  // no memory for it: those products read d_G
+  bool spare_alloc = false;  // what is being allocated only saves time, so nothing makes room for it
   // the same values in E2M1 for the FP32 drop-ins' products (k_fp4.cu), built at the first of them
   void* d_G4 = nullptr;
   bool g4_refused = false;  // no memory for it: those products run as the others
@@ -330,13 +334,20 @@ static int set_err(sg_ctx* c, int code, const char* fmt, ...) {
     if (r_ != SG_OK) return r_; \
   } while (0)
 
+static bool release_spares(sg_ctx* c);
+
 static int dev_alloc(sg_ctx* c, void** p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) bytes = 16;
-  if (c->budget && c->in_use + bytes > c->budget)
+  auto over = [&] { return c->budget && c->in_use + bytes > c->budget; };
+  cudaError_t e = over() ? cudaSuccess : cudaMalloc(p, bytes);
+  if ((over() || e != cudaSuccess) && release_spares(c)) {
+    cudaGetLastError();
+    e = over() ? cudaSuccess : cudaMalloc(p, bytes);
+  }
+  if (over())
     return set_err(c, SG_ERR_NOMEM, "HBM budget exceeded: %zu + %zu > %llu", (size_t)c->in_use,
                    bytes, (unsigned long long)c->budget);
-  cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaSuccess) {
     *p = nullptr;
     cudaGetLastError();
@@ -583,8 +594,9 @@ static int ensure_g(sg_ctx* c, int form) {
 static void free_g(sg_ctx* c) {
   dev_free(c, c->d_G);
   dev_free(c, c->d_G4);
-  c->d_G = c->d_G4 = nullptr;
-  c->g4_refused = false;
+  dev_free(c, c->d_Gp);
+  c->d_G = c->d_G4 = c->d_Gp = nullptr;
+  c->g4_refused = c->gp_refused = false;
 }
 
 extern "C" int sg_ctx_make_current(sg_ctx* c) {
@@ -1322,6 +1334,26 @@ static void fp4_free(sg_ctx* c) {
   w = Fp4Scratch{};
 }
 
+// Gives back the genotype copies that only save time (two-bit, E2M1), for an allocation that has to succeed.  Their
+// products run as the others from then on.
+static bool release_spares(sg_ctx* c) {
+  if (c->spare_alloc || (!c->d_Gp && !c->d_G4 && !c->d_Gk && !c->eng.f4.Vq)) return false;
+  dev_free(c, c->d_Gp);
+  dev_free(c, c->d_G4);
+  c->d_Gp = c->d_G4 = nullptr;
+  free_gk(c);
+  fp4_free(c);
+  c->gp_refused = c->g4_refused = c->gk_refused = true;
+  return true;
+}
+
+// While it lives, allocations are of such copies.
+struct SpareScope {
+  sg_ctx* c;
+  explicit SpareScope(sg_ctx* ctx) : c(ctx) { c->spare_alloc = true; }
+  ~SpareScope() { c->spare_alloc = false; }
+};
+
 // Scratch of the FP4 products over up to mg markers (a multiple of 128).
 static int fp4_scratch(sg_ctx* c, int64_t mg) {
   Engine& e = c->eng;
@@ -1341,12 +1373,32 @@ static int fp4_scratch(sg_ctx* c, int64_t mg) {
   return SG_OK;
 }
 
+// The two-bit genotype matrix of the subset-exact engine (an eighth of the BF16 one); false when there is no
+// memory (or budget) for it.
+static bool gpack_ready(sg_ctx* c) {
+  if (c->d_Gp) return true;
+  if (c->gp_refused) return false;
+  const SpareScope spare(c);
+  const int64_t each = gpack_bytes(c->mg, c->eng.np);
+  const std::string err = c->err;
+  if (dev_alloc(c, &c->d_Gp, (size_t)(2 * each)) != SG_OK) {
+    c->gp_refused = true;
+    c->err = err;
+    return false;
+  }
+  uint8_t* g = static_cast<uint8_t*>(c->d_Gp);
+  launch_gpack(c->d_codes, c->pitch, c->d_fill_all, c->m_bim, c->nn, c->mg, c->eng.np, g, g + each, c->stream);
+  c->launches += 2;
+  return true;
+}
+
 // The E2M1 genotype matrix of the subset-exact engine and the scratch of its FP4 products; false when there is
 // no memory (or budget) for them, and the products then run as the engine's others do.
 static bool fp4_ready(sg_ctx* c) {
   Engine& e = c->eng;
   if (c->d_G4 && e.f4.T && e.f4.mg >= c->mg) return true;
   if (c->g4_refused) return false;
+  const SpareScope spare(c);
   const int64_t mm = fp4_matrix_bytes(c->mg, c->nn);
   const bool build = !c->d_G4;
   auto all = [&]() -> int {
@@ -1408,6 +1460,7 @@ static int fp4_cohort_build(sg_ctx* c) {
 
 static bool fp4_cohort_ready(sg_ctx* c) {
   if (c->gk_refused) return false;
+  const SpareScope spare(c);
   const std::string err = c->err;
   const int64_t mg = round_up(c->m_qc, kRowTile);
   if ((!c->d_Gk && fp4_cohort_build(c) != SG_OK) || fp4_scratch(c, mg) != SG_OK) {
@@ -2425,12 +2478,15 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
     }
     launch_subset_prepare(e.Pf, np, e.d_gcols, npad, e.d_st, e.d_slots, e.winv, e.spart, vh, vl, c->stream);
     c->launches += 2;
-    cudaError_t err = tc_gemm_splitb(Gmm, mg, np, vh, vl, npad, e.Tm, mg, c->stream, false, 0);
+    const bool narrow = (tc_splitb_packed(np, npad) || tc_splitb_packed(mg, npad)) && gpack_ready(c);
+    const uint8_t* Pmm = narrow ? static_cast<const uint8_t*>(c->d_Gp) : nullptr;
+    const uint8_t* Psm = narrow ? Pmm + gpack_bytes(mg, np) : nullptr;
+    cudaError_t err = tc_gemm_splitb(Gmm, Pmm, mg, np, vh, vl, npad, e.Tm, mg, c->stream, false, 0);
     if (err != cudaSuccess) return set_err(c, SG_ERR_CUDA, "tcgen05 genotype GEMM (G'V): %s", cudaGetErrorString(err));
     launch_subset_scale(vh, vl, np, c->nn, e.d_gcols, npad, e.d_st, e.d_slots, e.max_w, e.Tm, mg, th, tl, e.spart,
                         c->stream);
     c->launches += e.max_w > 0 ? 3 : 2;
-    err = tc_gemm_splitb(Gsm, np, mg, th, tl, npad, e.Um, np, c->stream, false, 1);
+    err = tc_gemm_splitb(Gsm, Psm, np, mg, th, tl, npad, e.Um, np, c->stream, false, 1);
     if (err != cudaSuccess) return set_err(c, SG_ERR_CUDA, "tcgen05 genotype GEMM (G T'): %s", cudaGetErrorString(err));
     launch_subset_finalize(e.Um, np, c->nn, e.d_gcols, npad, e.d_st, e.d_slots, th, tl, mg, e.spart, e.winv, e.Yf,
                            c->stream);

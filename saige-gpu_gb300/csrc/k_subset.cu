@@ -127,6 +127,132 @@ void launch_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int
                                           static_cast<uint8_t*>(Gsm8));
 }
 
+// The same genotype values in two bits for the products of few columns (tc_packed_kernel), in both
+// layouts: (128 rows, stage of 128 elements of K) after (row block, stage), each [2 halves of 64
+// elements][128 rows][16 bytes].  A word holds 16 elements of K: rotated left by 2 i + 1, bits 7 and 14 say
+// of element 2 i, and bits 23 and 30 of element 2 i + 1, that it is 2 and that it is not 0.  Missing calls take the cohort fill; rows and elements past m and nn are zero.
+
+// 16 packed codes (00 two copies, 01 missing, 10 one, 11 none) to copies, in place
+__device__ __forceinline__ uint32_t pack_copies(uint32_t x, int fill, uint32_t valid) {
+  const uint32_t lo = x & 0x55555555u, hi = (x >> 1) & 0x55555555u, miss = lo & ~hi;
+  uint32_t one = hi & ~lo, two = ~(hi | lo) & 0x55555555u;
+  if (fill == 1) one |= miss;
+  if (fill == 2) two |= miss;
+  return (one & valid) | ((two & valid) << 1);
+}
+
+// The stored word of 16 elements whose copies are the fields of w, in the order of pack_order
+__device__ __forceinline__ uint32_t pack_flags(uint32_t w) {
+  const uint32_t two = (w >> 1) & 0x55555555u, any = (w | (w >> 1)) & 0x55555555u;
+  return two | __funnelshift_l(any, any, 7);
+}
+
+// 16 fields in element order to the order of pack_flags: even ones from field 3 down (and on from 15), odd ones
+// from 11 down
+__device__ __forceinline__ uint32_t pack_order(uint32_t x) {
+  uint32_t t = (x ^ (x >> 2)) & 0x0C0C0C0Cu;  // even fields to the low, odd fields to the high half
+  x ^= t ^ (t << 2);
+  t = (x ^ (x >> 4)) & 0x00F000F0u;
+  x ^= t ^ (t << 4);
+  t = (x ^ (x >> 8)) & 0x0000FF00u;
+  x ^= t ^ (t << 8);
+  x = __brev(x);  // reversed, the bits of a field turned back
+  x = ((x >> 1) & 0x55555555u) | ((x & 0x55555555u) << 1);
+  return __funnelshift_l(x, x, 8);
+}
+
+constexpr int kPackStages = 8;                 // stages of K per block of the marker rows
+constexpr int kPackPieces = 2 * kPackStages;   // 16-byte pieces (64 samples) of a row
+
+// Rows of markers: 256 bytes of codes of each of 128 markers, read 16 at a time, turned in shared memory and
+// written as whole stages.
+__global__ void __launch_bounds__(kThreads)
+gpack_mm_kernel(const uint8_t* __restrict__ codes, int64_t pitch, const int32_t* __restrict__ fill, int64_t m, int64_t nn,
+                int stages, uint4* __restrict__ out) {
+  __shared__ uint4 sp[kPackPieces][kRowTile + 1];
+  const int ks0 = blockIdx.x * kPackStages;
+  const int64_t rb = blockIdx.y;
+  for (int t = threadIdx.x; t < kRowTile * kPackPieces; t += kThreads) {
+    const int row = t / kPackPieces, q = t % kPackPieces;
+    const int64_t mk = rb * kRowTile + row, s0 = (int64_t)ks0 * kPackK + 64 * q;
+    uint32_t w[4] = {0, 0, 0, 0};
+    if (mk < m && s0 < nn) {  // rows are padded to 16 bytes, which is what is read
+      const uint4 x = *reinterpret_cast<const uint4*>(codes + mk * pitch + s0 / 4);
+      const int f = fill[mk];
+      const uint32_t c[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int64_t left = nn - (s0 + 16 * i);
+        const uint32_t valid = left >= 16 ? 0x55555555u : left <= 0 ? 0u : 0x55555555u & ((1u << (2 * left)) - 1u);
+        w[i] = pack_flags(pack_order(pack_copies(c[i], f, valid)));
+      }
+    }
+    sp[q][row] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < kRowTile * kPackPieces; t += kThreads) {
+    const int q = t / kRowTile, row = t % kRowTile, ks = ks0 + q / 2;
+    if (ks < stages) out[((rb * stages + ks) * 2 + (q & 1)) * kRowTile + row] = sp[q][row];
+  }
+}
+
+// Rows of samples: block = one stage (128 markers) x 512 samples; a thread turns 16 markers x 16 samples
+// of codes in registers (a transposition of 16 x 16 two-bit fields).
+__global__ void __launch_bounds__(kThreads)
+gpack_sm_kernel(const uint8_t* __restrict__ codes, int64_t pitch, const int32_t* __restrict__ fill, int64_t m, int64_t nn,
+                int stages, int64_t row_blocks, uint4* __restrict__ out) {
+  // four row blocks of two halves, rows of four words padded per 16 rows: a warp's stores meet every bank once
+  constexpr int kHalfW = 4 * kRowTile + 4 * (kRowTile / 16), kBlockW = 2 * kHalfW + 1;
+  __shared__ uint32_t so[4 * kBlockW];
+  const int ks = blockIdx.x;
+  const int64_t rb0 = 4 * (int64_t)blockIdx.y;
+  const int sw = threadIdx.x & 31, mg = threadIdx.x >> 5;
+  const int64_t s0 = rb0 * kRowTile + 16 * sw;
+  const int64_t left = nn - s0;
+  const uint32_t valid = left >= 16 ? 0x55555555u : left <= 0 ? 0u : 0x55555555u & ((1u << (2 * left)) - 1u);
+  uint32_t w[16];
+#pragma unroll
+  for (int p = 0; p < 16; ++p) {  // the element of field p in the order of pack_flags
+    const int64_t mk = (int64_t)ks * kPackK + 16 * mg + (p < 4 ? 2 * (3 - p) : p < 12 ? 2 * (11 - p) + 1 : 2 * (19 - p));
+    // pitch is a multiple of 16, so a word that starts inside a row ends there
+    w[p] = mk < m && left > 0 ? pack_copies(*reinterpret_cast<const uint32_t*>(codes + mk * pitch + s0 / 4), fill[mk], valid) : 0u;
+  }
+#pragma unroll
+  for (int d = 8; d > 0; d >>= 1) {  // swap the off-diagonal d x d blocks of fields
+    const uint32_t mask = d == 8 ? 0x0000FFFFu : d == 4 ? 0x00FF00FFu : d == 2 ? 0x0F0F0F0Fu : 0x33333333u;
+#pragma unroll
+    for (int p = 0; p < 16; ++p)
+      if (!(p & d)) {
+        const uint32_t t = ((w[p] >> (2 * d)) ^ w[p + d]) & mask;
+        w[p + d] ^= t;
+        w[p] ^= t << (2 * d);
+      }
+  }
+  const int base = (sw >> 3) * kBlockW + (mg >> 2) * kHalfW + (sw & 7) * (4 * 16 + 4) + (mg & 3);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) so[base + 4 * i] = pack_flags(w[i]);
+  __syncthreads();
+  for (int t = threadIdx.x; t < 4 * 2 * kRowTile; t += kThreads) {
+    const int row = t % kRowTile, half = (t / kRowTile) & 1, b = t / (2 * kRowTile);
+    if (rb0 + b >= row_blocks) break;
+    const uint32_t* p = so + b * kBlockW + half * kHalfW + 4 * row + 4 * (row >> 4);
+    out[((((rb0 + b) * stages + ks) * 2) + half) * kRowTile + row] = make_uint4(p[0], p[1], p[2], p[3]);
+  }
+}
+
+int64_t gpack_bytes(int64_t mg, int64_t np) { return mg * np / 4; }
+
+// mg markers x np samples, multiples of 128, each way gpack_bytes()
+void launch_gpack(const uint8_t* codes, int64_t pitch, const int32_t* fill, int64_t m, int64_t nn, int64_t mg,
+                  int64_t np, void* Gmm, void* Gsm, cudaStream_t s) {
+  const int sn = (int)(np / kPackK), sm = (int)(mg / kPackK);
+  gpack_mm_kernel<<<dim3((unsigned)((sn + kPackStages - 1) / kPackStages), (unsigned)(mg / kRowTile)), kThreads, 0, s>>>(
+      codes, pitch, fill, m, nn, sn, static_cast<uint4*>(Gmm));
+  const int64_t rs = np / kRowTile;
+  gpack_sm_kernel<<<dim3((unsigned)sm, (unsigned)((rs + 3) / 4)), kThreads, 0, s>>>(codes, pitch, fill, m, nn, sm, rs,
+                                                                                static_cast<uint4*>(Gsm));
+}
+
 // A subset's GRM tables from its per-marker QC records, as setgeno over the subset builds them
 // (the LUT's 2p and 1/sd: FIT.cpp:152-159): for each GRM marker of the subset, d' = (1/sd')^2,
 // 2p' (in FP32 as the reference's LUT, and in FP64 from the allele count: the mean genotype), and lut4 = d' (g - 2p')^2 for the four packed codes (00 -> 2, 01 -> the subset's own fill,

@@ -497,6 +497,231 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   }
 }
 
+// ---------------------------------------------------------------- few columns, two-bit genotypes
+// D = A (Bh + Bl)^T as kSplitB above, for few columns, where that form is bound by A's stream from HBM: A
+// (genotypes 0, 1, 2) is held in two bits and widened to BF16 on the way into TMEM, from where the MMA
+// takes it.  Products, their order in an accumulator and the drains are those of kSplitB (16 elements of K per
+// MMA, high half then low, an accumulator per drain length), so the results are the same bits.
+//
+// A stage is 128 elements of K: 4 KB of packed rows (one contiguous read) and two 128-byte boxes of each
+// half of B.  kExp warps (one row a thread, sets of four taking stages in turn) widen a stage into one of
+// kBufs buffers of 64 TMEM columns; a word is eight columns, one rotation and one mask each, which give 2 g: the sums
+// are twice kSplitB's, exactly, and halved on the way out.  Then four warps drain (one quadrant each, every column), one loads and one issues the
+// MMAs.  Two CTAs share an SM up to 64 columns.
+//
+// What bounds it: at 64 and 96 columns the MMAs and the operands' way from L2 into shared memory, at 32 the
+// hand-overs of a stage from warp to warp (two CTAs an SM and, at 32 columns, two sets of widening warps on
+// alternate stages hide part of them).  Mean of the two GEMMs of a product at N = 50,000, M = 100,000: 32 columns
+// 2.06 to 0.66 ms, 64 2.09 to 0.93 (BF16 G from HBM at 4.9 TB/s before).
+constexpr int kPackABytes = kTileM * kPackK / 4;  // 4,096: a row block's two-bit genotypes of one stage
+
+__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate));
+}
+
+// 32 TMEM columns (64 elements of this thread's row) from four words of two-bit genotypes: column 8 w + i is
+// word w rotated left by 2 i + 1 under a mask, which leaves 2 g in BF16 (0, 0x4000, 0x4080) in either half
+__device__ __forceinline__ void tmem_st_bf16(uint32_t taddr, const uint4& g) {
+  const uint32_t w[4] = {g.x, g.y, g.z, g.w};
+  uint32_t o[32];
+#pragma unroll
+  for (int c = 0; c < 32; ++c) o[c] = __funnelshift_l(w[c >> 3], w[c >> 3], 2 * (c & 7) + 1) & 0x40804080u;
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]),
+        "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15]), "r"(o[16]), "r"(o[17]),
+        "r"(o[18]), "r"(o[19]), "r"(o[20]), "r"(o[21]), "r"(o[22]), "r"(o[23]), "r"(o[24]), "r"(o[25]), "r"(o[26]),
+        "r"(o[27]), "r"(o[28]), "r"(o[29]), "r"(o[30]), "r"(o[31]) : "memory");
+}
+
+template <int BN, int S, int kBufs, int kCtas, int kExp>
+__global__ void __launch_bounds__(32 * (kExp + 6), kCtas)
+tc_packed_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMap mapB,
+                 const __grid_constant__ CUtensorMap mapB2, int stages, int drain, int ncolt, float* __restrict__ D,
+                 int64_t ldd) {
+  constexpr int kHalf = BN * 2 * kPackK;               // bytes of one half of B per stage
+  constexpr int kStage = kPackABytes + 2 * kHalf;
+  constexpr int kACols = kPackK / 2;                   // TMEM columns of a stage of A
+  constexpr uint32_t kABase = 2 * BN, kTmem = 512 / kCtas;
+  constexpr uint32_t kIdesc = make_idesc(1u, kTileM, BN);
+  static_assert(kABase + kBufs * kACols <= kTmem, "two accumulators and the A buffers fit the TMEM allocation");
+  constexpr int kLoadWarp = kExp + 4, kIssueWarp = kExp + 5, kGroups = kExp / 4;
+  static_assert(kExp % 4 == 0, "a warp reaches the TMEM lanes of its quarter of a warpgroup");
+  static_assert(S >= kBufs, "an A buffer's release is its stage's");
+
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * kStage);
+  uint64_t* empty = full + S;         // the MMAs have read a stage, and with it its A buffer
+  uint64_t* t_full = empty + S;       // [kBufs] an A buffer is written
+  uint64_t* acc_full = t_full + kBufs;
+  uint64_t* acc_empty = acc_full + 2;
+  uint64_t* mma_done = acc_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rt = blockIdx.x / ncolt, bt = blockIdx.x - rt * ncolt;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < kBufs; ++b) mbar_init(&t_full[b], 4);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 4);
+    }
+    mbar_init(mma_done, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == kIssueWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmem)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+
+  if (warp == kLoadWarp) {
+    if (elect_one()) {
+      const uint8_t* a = A + (int64_t)rt * stages * kPackABytes;
+      int issued = 0;
+      for (int kb = 0; kb < stages; ++kb) {
+        const int s = kb % S;
+        if (!mbar_wait(&empty[s], ((uint32_t)(kb / S) & 1u) ^ 1u, 1, abort_flag, &g_tc_error)) break;
+        uint8_t* st = smem + s * kStage;
+        mbar_expect_tx(&full[s], (uint32_t)kStage);
+        bulk_load(st, a + (int64_t)kb * kPackABytes, kPackABytes, &full[s]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          tma_load_2d(st + kPackABytes + u * (kHalf / 2), &mapB, &full[s], kb * kPackK + 64 * u, bt * BN);
+          tma_load_2d(st + kPackABytes + kHalf + u * (kHalf / 2), &mapB2, &full[s], kb * kPackK + 64 * u, bt * BN);
+        }
+        issued = kb + 1;
+      }
+      // after an abort: the loads in flight land before the shared memory is given up
+      if (*abort_flag)
+        for (int kb = issued > S ? issued - S : 0; kb < issued; ++kb)
+          mbar_wait_teardown(&full[kb % S], (uint32_t)(kb / S) & 1u);
+    }
+  } else if (warp == kIssueWarp) {
+    if (elect_one()) {
+      for (int kb = 0, ch = 0, kin = 0; kb < stages; ++kb) {
+        const int s = kb % S, t = kb % kBufs, ab = ch & 1;
+        if (kin == 0 && !mbar_wait(&acc_empty[ab], ((uint32_t)(ch >> 1) & 1u) ^ 1u, 5, abort_flag, &g_tc_error)) break;
+        if (!mbar_wait(&full[s], (uint32_t)(kb / S) & 1u, 2, abort_flag, &g_tc_error) ||
+            !mbar_wait(&t_full[t], (uint32_t)(kb / kBufs) & 1u, 6, abort_flag, &g_tc_error))
+          break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t dacc = tmem + (uint32_t)(ab * BN), a0 = tmem + kABase + (uint32_t)(t * kACols);
+        const uint32_t b0 = smem_u32(smem + s * kStage) + kPackABytes;
+#pragma unroll
+        for (int k = 0; k < kPackK / 16; ++k) {
+          const uint32_t kbo = (uint32_t)((k >> 2) * (kHalf / 2) + 32 * (k & 3));
+          umma_ts(dacc, a0 + 8u * k, smem_desc_sw128(b0 + kbo), kIdesc, (kin > 0 || k > 0) ? 1u : 0u);
+          umma_ts(dacc, a0 + 8u * k, smem_desc_sw128(b0 + kHalf + kbo), kIdesc, 1u);
+        }
+        umma_commit<false>(smem_u32(&empty[s]));
+        if (++kin == drain || kb == stages - 1) {
+          umma_commit<false>(smem_u32(&acc_full[ab]));
+          kin = 0;
+          ++ch;
+        }
+      }
+      umma_commit<false>(smem_u32(mma_done));
+      mbar_wait_teardown(mma_done, 0u);
+    }
+  } else if (warp < kExp) {
+    const int row = threadIdx.x & (kTileM - 1);
+    uint4 g0, g1;
+    auto fetch = [&](int kb) -> int {
+      const int s = kb % S;
+      if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (uint32_t)(kb / S) & 1u, 4, abort_flag, &g_tc_error))) return 0;
+      const uint4* p = reinterpret_cast<const uint4*>(smem + s * kStage) + row;
+      g0 = p[0];
+      g1 = p[kTileM];
+      return 1;
+    };
+    int kb = warp >> 2, go = kb < stages && fetch(kb);
+    for (; go && kb < stages; kb += kGroups) {
+      const int t = kb % kBufs;
+      if (kb >= kBufs) {  // the buffer's last stage
+        const int u = kb - kBufs;
+        go = __all_sync(0xffffffffu, mbar_wait(&empty[u % S], (uint32_t)(u / S) & 1u, 7, abort_flag, &g_tc_error));
+        if (!go) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      const uint32_t ta = tl + kABase + (uint32_t)(t * kACols);
+      tmem_st_bf16(ta, g0);
+      tmem_st_bf16(ta + 32, g1);
+      if (kb + kGroups < stages) go = fetch(kb + kGroups);  // while the stores are on their way
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&t_full[t]);
+    }
+  } else {
+    float sum[BN];
+#pragma unroll
+    for (int j = 0; j < BN; ++j) sum[j] = 0.0f;
+    const int nchunks = (stages + drain - 1) / drain;
+    int go = 1;
+    for (int ch = 0; ch < nchunks; ++ch) {
+      const int ab = ch & 1;
+      if (lane == 0) go = mbar_wait(&acc_full[ab], (uint32_t)(ch >> 1) & 1u, 3, abort_flag, &g_tc_error) && !*abort_flag;
+      go = __shfl_sync(0xffffffffu, go, 0);
+      __syncwarp();
+      if (!go) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < BN; c += 16) {
+        uint32_t v[16];
+        tmem_ld16(tl + (uint32_t)(ab * BN + c), v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) sum[c + j] += __uint_as_float(v[j]);
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[ab]);
+    }
+    if (go) {
+      float* o = D + (int64_t)bt * BN * ldd + (int64_t)rt * kTileM + (warp & 3) * 32 + lane;
+#pragma unroll
+      for (int j = 0; j < BN; ++j) o[j * ldd] = 0.5f * sum[j];
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == kIssueWarp)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmem) : "memory");
+}
+
+template <int BN, int S, int kBufs, int kCtas, int kExp>
+cudaError_t launch_packed(const uint8_t* A, const CUtensorMap& b, const CUtensorMap& b2, int64_t rows, int stages, int drain,
+                          int ncolt, float* D, int64_t ldd, cudaStream_t s) {
+  auto k = tc_packed_kernel<BN, S, kBufs, kCtas, kExp>;
+  constexpr size_t sm = (size_t)S * (kPackABytes + 4 * BN * kPackK) + 1024 + 256;
+  static_assert((sm + 1024) * kCtas <= 233472 && 2 * S + kBufs + 6 <= 31, "kCtas CTAs' stages and barriers fit the SM");
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  k<<<(unsigned)(rows / kTileM * ncolt), 32 * (kExp + 6), sm, s>>>(A, b, b2, stages, drain, ncolt, D, ldd);
+  return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------- host side
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -920,13 +1145,19 @@ int tc_gemm_tile_n(int64_t ncols, int set) {
   return set == kTilesSplitBF16 ? 16 : 32;
 }
 
-// CTA pairs for a subset-exact genotype GEMM over ncols columns: measured at N = 100k, M = 150k,
-// 256-byte K stages, pairs took 512 columns from 49.7 to 32.8 ms and 1024 from 89.4 to 61.8 ms,
-// and were 5-12% slower up to 128 columns, where the launch streams G from HBM.
+// Few columns stay off CTA pairs and take their genotypes in two bits (tc_packed_kernel).  Measured per product
+// (two GEMMs) at N = 50,000, M = 100,000, two-bit form against CTA pairs on the BF16 one: 32 columns 1.38
+// against 3.00 ms, 64 1.98 against 3.15, 96 2.72 against 3.23, but 128 4.12 against 3.57 (and there at
+// N = 20,000, M = 30,000 0.74 against 0.64).  Single CTAs on the BF16 form were the slowest at each width.
+constexpr int kPackMaxCols = 96;
+
+// CTA pairs for a subset-exact genotype GEMM over ncols columns: every width without the two-bit form (at
+// 160 columns 3.82 against 5.10 ms; at N = 100k, M = 150k, 256-byte K stages, pairs took 512 columns from
+// 49.7 to 32.8 ms and 1024 from 89.4 to 61.8 ms).
 static bool subset_pair(int64_t ncols) {
   for (const GrmvChoice& b : g_subset_plan)
     if (ncols <= b.max_cols) return b.pair != 0;
-  return g_opt[kTcSubsetPair] == 2 ? ncols > 160 : g_opt[kTcSubsetPair] != 0;
+  return g_opt[kTcSubsetPair] == 2 ? ncols > kPackMaxCols : g_opt[kTcSubsetPair] != 0;
 }
 
 static int subset_slice(int64_t ncols) {
@@ -963,7 +1194,8 @@ int64_t tc_grmv_padded_cols(int64_t ncols32, int64_t cap, int64_t np, int set, i
     const int64_t tiles = nrt * (padded / bn);
     const int64_t waves = (tiles + slots - 1) / slots;
     const double eff = (double)tiles / (double)(waves * slots);
-    const double cost = (double)padded * ((double)kATileBytes / bn + (double)kRowBytes / (pair ? 2 : 1)) / eff;
+    const bool packed = set == kTilesSplitB && !pair && bn <= kPackMaxCols;  // an eighth of the A bytes
+    const double cost = (double)padded * ((double)kATileBytes / (packed ? 8 : 1) / bn + (double)kRowBytes / (pair ? 2 : 1)) / eff;
     if (cost < best) {
       best = cost;
       best_cols = padded;
@@ -1176,18 +1408,36 @@ cudaError_t tc_gemm_bf16x3(const void* Kh, const void* Kl, int64_t np, const voi
   return check ? check_error_flag(s) : cudaSuccess;
 }
 
+bool tc_splitb_packed(int64_t kdim, int64_t ncols) {
+  return !subset_pair(ncols) && tc_gemm_tile_n(ncols, kTilesSplitB) <= kPackMaxCols && kdim % kPackK == 0 &&
+         g_opt[kTcDrainBytes] % (2 * kPackK) == 0;
+}
+
 // D = A (Bh + Bl)^T: A (rows x kdim) exact in BF16 (genotype values), B as BF16 high + low halves
 // (ncols x kdim), two products per K step into the drained TMEM accumulators; D RHS-major (column j
 // of the product is row j of D, leading dimension ldd).  K slices of 128 bytes by default (each
 // 128-byte row segment of A is a whole DRAM burst line; measured at N = 100k, M = 150k they took
 // 32-128 columns from 23-24 ms to 16 ms and, on CTA pairs, 512 columns from 54 to 36.5 ms), or
 // 64 bytes (twice the stages); as many stages as fit.
-cudaError_t tc_gemm_splitb(const void* A, int64_t rows, int64_t kdim, const void* Bh, const void* Bl,
-                           int64_t ncols, float* D, int64_t ldd, cudaStream_t s, bool check, int site) {
+cudaError_t tc_gemm_splitb(const void* A, const void* A2bit, int64_t rows, int64_t kdim, const void* Bh,
+                           const void* Bl, int64_t ncols, float* D, int64_t ldd, cudaStream_t s, bool check, int site) {
   if (rows % kTileM != 0 || kdim % 64 != 0 || ncols % 32 != 0 || ncols <= 0 || !A || !Bh || !Bl || site < 0 ||
       site > 1)
     return cudaErrorInvalidValue;
   const int BN = tc_gemm_tile_n(ncols, kTilesSplitB);
+  if (A2bit && tc_splitb_packed(kdim, ncols)) {
+    CUtensorMap b, b2;
+    const uint64_t rb = (uint64_t)kdim * 2;
+    if (!make_map(&b, Bh, false, kdim, ncols, rb, BN) || !make_map(&b2, Bl, false, kdim, ncols, rb, BN))
+      return cudaErrorInvalidValue;
+    const uint8_t* a = static_cast<const uint8_t*>(A2bit);
+    const int stages = (int)(kdim / kPackK), ncolt = (int)(ncols / BN), dr = drain_stages(2 * kPackK);
+    const cudaError_t e = BN == 32 ? launch_packed<32, 5, 3, 2, 8>(a, b, b2, rows, stages, dr, ncolt, D, ldd, s)
+                          : BN == 64 ? launch_packed<64, 3, 2, 2, 4>(a, b, b2, rows, stages, dr, ncolt, D, ldd, s)
+                                     : launch_packed<96, 4, 4, 1, 4>(a, b, b2, rows, stages, dr, ncolt, D, ldd, s);
+    if (e != cudaSuccess) return e;
+    return check ? check_error_flag(s) : cudaSuccess;
+  }
   const bool pair = subset_pair(ncols);
   int RB = splitb_stage_bytes(subset_slice(ncols), BN, pair);
   while (RB > 128 && kdim % (RB / 2) != 0) RB /= 2;  // whole stages over K

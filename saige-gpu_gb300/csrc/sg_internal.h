@@ -137,9 +137,12 @@ int tc_get_subset_plan(int32_t* max_cols, int32_t* pair, int32_t* slice, int cap
 // the subset-exact genotype GEMMs (multiples of 32)
 enum { kTilesPlain = 0, kTilesSplitTF32 = 1, kTilesSplitBF16 = 2, kTilesSplitB = 3 };
 // D (ncols x ldd, RHS-major) = A (rows x kdim, exact BF16) (Bh + Bl)^T (ncols x kdim BF16 halves).
+// A2bit (may be null): the same A as launch_gpack lays it out, used where tc_splitb_packed says so
+// (then A itself is not read).
 // site (0 or 1): which of two call sites queued back to back on one stream (own tile tables).
-cudaError_t tc_gemm_splitb(const void* A, int64_t rows, int64_t kdim, const void* Bh, const void* Bl,
+cudaError_t tc_gemm_splitb(const void* A, const void* A2bit, int64_t rows, int64_t kdim, const void* Bh, const void* Bl,
                            int64_t ncols, float* D, int64_t ldd, cudaStream_t s, bool check, int site);
+bool tc_splitb_packed(int64_t kdim, int64_t ncols);
 // The same with FP16 high halves and E4M3 low halves (A in FP16 and in E4M3, kdim a multiple of 128)
 cudaError_t tc_gemm_splitb8(const void* A, const void* A8, int64_t rows, int64_t kdim, const void* Bh,
                             const void* Bl8, int64_t ncols, float* D, int64_t ldd, cudaStream_t s, bool check,
@@ -223,6 +226,11 @@ struct SubsetSlot {
 // form 0: BF16 G (Gmm16, Gsm16); form 1: FP16 G (Gmm16, Gsm16) and E4M3 G (Gmm8, Gsm8)
 void launch_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int64_t m, int64_t nn, int64_t mg,
                    int64_t np, int form, void* Gmm16, void* Gsm16, void* Gmm8, void* Gsm8, cudaStream_t s);
+// G in two bits, both layouts (gpack_bytes each), in stages of kPackK elements of K
+constexpr int kPackK = 128;
+int64_t gpack_bytes(int64_t mg, int64_t np);
+void launch_gpack(const uint8_t* codes, int64_t pitch, const int32_t* fill, int64_t m, int64_t nn, int64_t mg,
+                  int64_t np, void* Gmm, void* Gsm, cudaStream_t s);
 // the subset's d', 2p', diagonal table, fill-change list and counts (nflip, M') from its QC records;
 // flag: mg bytes of scratch, flips / dfill: room for m entries, counts: 2 int64 on the device;
 // markers ex_lo..ex_hi are left out of the subset's GRM (none when ex_lo > ex_hi)

@@ -1,0 +1,69 @@
+"""Products of few columns through two-bit genotypes (csrc/k_tc.cu, tc_packed_kernel) against the BF16 genotype matrix
+on CTA pairs: the same products in the same order, so the same bits."""
+import numpy as np
+import pytest
+
+from saigegpu import MV_FP32_SIMT, MV_SUBSET_EXACT, TC_SUBSET_PAIR, Context, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,m", [(40, 30), (128, 128), (129, 257), (511, 1300), (1025, 640)])
+def test_same_bits_as_bf16(gpu_ctx, n, m):
+    """One to nine stages, fewer and more than the kernel has buffers; rows, samples and markers past a tile."""
+    ctx = gpu_ctx
+    bed, _ = synth.synth_bed(40 + n, n, m, 0.05)
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    mask = np.random.default_rng(n).uniform(size=n) > 0.2  # fills that differ from the cohort's
+    try:
+        ctx.set_matvec_mode(MV_SUBSET_EXACT)
+        ctx.engine_reserve(128, 1)
+        ctx.engine_set_pheno(0, np.ones(n), np.array([1.0, 0.5]), mask)
+        for k in (1, 33, 64, 65, 96):
+            V = np.random.default_rng(k).standard_normal((n, k)) * 10.0 ** np.linspace(-18, 18, k)
+            V[~mask] = 0.0
+            out = []
+            for pair in (0, 1):
+                ctx.set_tc_option(TC_SUBSET_PAIR, pair)
+                ids = [int(i) for i in ctx.engine_submit(0, 1, V)]
+                got = {}
+                for _ in range(1000):
+                    if len(got) == k:
+                        break
+                    ctx.engine_run()
+                    got.update({i: r[0] for i in ids if i not in got and (r := ctx.engine_try_fetch(i)) is not None})
+                out.append(np.column_stack([got[i] for i in ids]))
+            np.testing.assert_array_equal(out[0], out[1])
+            assert np.isfinite(out[0]).all() and np.abs(out[0]).max(0).min() > 0
+    finally:
+        ctx.set_tc_option(TC_SUBSET_PAIR, 2)
+        ctx.set_matvec_mode(MV_FP32_SIMT)
+
+
+def test_gives_way_to_other_memory():
+    """Under a budget the two-bit copy is left out, or given back for what has to be allocated."""
+    n, m = 500, 900
+    bed, _ = synth.synth_bed(9, n, m, 0.02)
+    V = np.random.default_rng(1).standard_normal((n, 8))
+
+    def run(budget, grow=True):
+        with Context(0, budget) as ctx:
+            ctx.setgeno(bed, n, m)
+            ctx.set_matvec_mode(MV_SUBSET_EXACT)
+            ctx.engine_reserve(128, 1)
+            a = ctx.grm_matmul(V)
+            used1 = ctx.bytes_in_use()
+            if grow:
+                ctx.engine_reserve(256, 1)
+            b = ctx.grm_matmul(V)
+            return a, b, used1, ctx.bytes_in_use()
+
+    a, b, used1, used2 = run(0)
+    packed = 2 * 1024 * 512 // 4
+    c = run(used1 - packed, False)  # left out
+    d = run(used2 - packed)  # taken, then given back or left out for the larger engine
+    for o in (b, c[0], d[0], d[1]):
+        np.testing.assert_array_equal(o, a)
+    assert c[3] == used1 - packed
+    assert d[2] == used1 and d[3] == used2 - packed
