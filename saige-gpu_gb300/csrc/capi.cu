@@ -1418,7 +1418,13 @@ static bool fp4_ready(sg_ctx* c) {
   }
   if (build) {
     uint8_t* g = static_cast<uint8_t*>(c->d_G4);
-    launch_fp4_gbuild(c->d_codes, c->pitch, c->d_fill_all, c->m_bim, c->nn, g, g + mm, c->stream);
+    if (launch_fp4_gbuild(c->d_codes, c->pitch, c->d_fill_all, c->m_bim, c->nn, g, g + mm, c->stream) != cudaSuccess) {
+      fp4_free(c);
+      dev_free(c, c->d_G4);
+      c->d_G4 = nullptr;
+      c->g4_refused = true;
+      return false;
+    }
     c->launches += 2;
   }
   return true;
@@ -1453,7 +1459,7 @@ static int fp4_cohort_build(sg_ctx* c) {
   SG_CUDA(c, cudaMemcpyAsync(c->d_gk_p2d, p2d.data(), mg * 8, cudaMemcpyHostToDevice, c->stream));
   SG_CUDA(c, cudaMemcpyAsync(c->d_gk_slot, &sl, sizeof(sl), cudaMemcpyHostToDevice, c->stream));
   uint8_t* g = static_cast<uint8_t*>(c->d_Gk);
-  launch_fp4_gbuild(c->d_packed, c->pitch, nullptr, m, c->nn, g, g + mm, c->stream);
+  SG_CUDA(c, launch_fp4_gbuild(c->d_packed, c->pitch, nullptr, m, c->nn, g, g + mm, c->stream));
   SG_LAUNCHED(c, 2);
   return sync(c);  // the tables above are on this function's stack
 }

@@ -17,6 +17,7 @@
 // Every kernel below reduces in a fixed order, so a column's product does not depend on which
 // other columns share the step.
 #include "sg_internal.h"
+#include "geno_bits.cuh"
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -132,15 +133,6 @@ void launch_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int
 // elements][128 rows][16 bytes].  A word holds 16 elements of K: rotated left by 2 i + 1, bits 7 and 14 say
 // of element 2 i, and bits 23 and 30 of element 2 i + 1, that it is 2 and that it is not 0.  Missing calls take the cohort fill; rows and elements past m and nn are zero.
 
-// 16 packed codes (00 two copies, 01 missing, 10 one, 11 none) to copies, in place
-__device__ __forceinline__ uint32_t pack_copies(uint32_t x, int fill, uint32_t valid) {
-  const uint32_t lo = x & 0x55555555u, hi = (x >> 1) & 0x55555555u, miss = lo & ~hi;
-  uint32_t one = hi & ~lo, two = ~(hi | lo) & 0x55555555u;
-  if (fill == 1) one |= miss;
-  if (fill == 2) two |= miss;
-  return (one & valid) | ((two & valid) << 1);
-}
-
 // The stored word of 16 elements whose copies are the fields of w, in the order of pack_order
 __device__ __forceinline__ uint32_t pack_flags(uint32_t w) {
   const uint32_t two = (w >> 1) & 0x55555555u, any = (w | (w >> 1)) & 0x55555555u;
@@ -182,9 +174,7 @@ gpack_mm_kernel(const uint8_t* __restrict__ codes, int64_t pitch, const int32_t*
       const uint32_t c[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int64_t left = nn - (s0 + 16 * i);
-        const uint32_t valid = left >= 16 ? 0x55555555u : left <= 0 ? 0u : 0x55555555u & ((1u << (2 * left)) - 1u);
-        w[i] = pack_flags(pack_order(pack_copies(c[i], f, valid)));
+        w[i] = pack_flags(pack_order(pack_copies(c[i], f, valid_fields(nn - (s0 + 16 * i)))));
       }
     }
     sp[q][row] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -209,7 +199,7 @@ gpack_sm_kernel(const uint8_t* __restrict__ codes, int64_t pitch, const int32_t*
   const int sw = threadIdx.x & 31, mg = threadIdx.x >> 5;
   const int64_t s0 = rb0 * kRowTile + 16 * sw;
   const int64_t left = nn - s0;
-  const uint32_t valid = left >= 16 ? 0x55555555u : left <= 0 ? 0u : 0x55555555u & ((1u << (2 * left)) - 1u);
+  const uint32_t valid = valid_fields(left);
   uint32_t w[16];
 #pragma unroll
   for (int p = 0; p < 16; ++p) {  // the element of field p in the order of pack_flags
@@ -217,17 +207,7 @@ gpack_sm_kernel(const uint8_t* __restrict__ codes, int64_t pitch, const int32_t*
     // pitch is a multiple of 16, so a word that starts inside a row ends there
     w[p] = mk < m && left > 0 ? pack_copies(*reinterpret_cast<const uint32_t*>(codes + mk * pitch + s0 / 4), fill[mk], valid) : 0u;
   }
-#pragma unroll
-  for (int d = 8; d > 0; d >>= 1) {  // swap the off-diagonal d x d blocks of fields
-    const uint32_t mask = d == 8 ? 0x0000FFFFu : d == 4 ? 0x00FF00FFu : d == 2 ? 0x0F0F0F0Fu : 0x33333333u;
-#pragma unroll
-    for (int p = 0; p < 16; ++p)
-      if (!(p & d)) {
-        const uint32_t t = ((w[p] >> (2 * d)) ^ w[p + d]) & mask;
-        w[p + d] ^= t;
-        w[p] ^= t << (2 * d);
-      }
-  }
+  transpose_fields(w);
   const int base = (sw >> 3) * kBlockW + (mg >> 2) * kHalfW + (sw & 7) * (4 * 16 + 4) + (mg & 3);
 #pragma unroll
   for (int i = 0; i < 16; ++i) so[base + 4 * i] = pack_flags(w[i]);

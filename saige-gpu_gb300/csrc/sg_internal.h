@@ -277,8 +277,8 @@ int64_t fp4_matrix_bytes(int64_t rows, int64_t k);  // G in E2M1 stages: rows pa
 int64_t fp4_digit_bytes(int64_t cols, int64_t k);   // room for cols columns' digits, whatever the tile
 // G with rows of markers (m x nn) and with rows of samples (nn x m), missing calls at the cohort fill (fill may
 // be null when there are none)
-void launch_fp4_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int64_t m, int64_t nn, void* Gmm,
-                       void* Gsm, cudaStream_t s);
+cudaError_t launch_fp4_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int64_t m, int64_t nn, void* Gmm,
+                              void* Gsm, cudaStream_t s);
 // columns per tile for a launch over ncols columns (pad ncols to a multiple of it)
 int fp4_tile_cols(int64_t ncols);
 // Scratch of one subset-exact product over up to ``cap`` columns (cap counts the padding columns)
