@@ -583,7 +583,7 @@ static int ensure_g(sg_ctx* c, int form) {
   uint8_t* g8 = reinterpret_cast<uint8_t*>(g16 + 2 * mg * np);
   launch_gbuild(c->d_codes, c->pitch, c->d_fill_all, c->m_bim, c->nn, mg, np, form, g16, g16 + mg * np,
                 form ? g8 : nullptr, form ? g8 + mg * np : nullptr, c->stream);
-  SG_LAUNCHED(c, 1);
+  SG_LAUNCHED(c, 2);
   SG_CUDA(c, cudaEventRecord(c->tev[1], c->stream));
   SG_TRY(sync(c));
   c->t_build[3] = ev_ms(c->tev[0], c->tev[1]);

@@ -85,47 +85,76 @@ __device__ __forceinline__ uint16_t g_bf16(int g) { return g == 0 ? 0x0000u : g 
 __device__ __forceinline__ uint16_t g_f16(int g) { return g == 0 ? 0x0000u : g == 1 ? 0x3C00u : 0x4000u; }
 __device__ __forceinline__ uint8_t g_e4m3(int g) { return g == 0 ? 0x00u : g == 1 ? 0x38u : 0x40u; }
 
-// G in both layouts from the cohort's packed codes (missing calls kept as 01): block = 64 markers x
-// 128 samples staged through shared memory, written coalesced along samples (marker-major G_mm,
-// mg x np) and along markers (sample-major G_sm, np x mg).  Missing calls take the cohort fill;
-// rows and columns past m and nn are zero.
+// G in both layouts from the cohort's packed codes (missing calls kept as 01), 16 codes at a time: marker-major
+// G_mm (mg x np) and sample-major G_sm (np x mg).  Missing calls take the cohort fill; rows and columns past m and nn are
+// zero.  Bound by the bytes written.  At N = 100,000, M = 150,000 (60 GB in BF16): the rows
+// of markers 9.1 ms and the rows of samples 11.2, against 39.7 for both a code at a time.
 // form 0: BF16 G in both layouts (Gmm16, Gsm16 hold BF16 bits); form 1: FP16 G in both layouts and
 // E4M3 G in both layouts (Gmm8, Gsm8), for the FP16-high / E4M3-low products.
-__global__ void gbuild_kernel(const uint8_t* __restrict__ codes, int64_t pitch, const int32_t* __restrict__ fill,
-                              int64_t m, int64_t nn, int64_t mg, int64_t np, int form, uint16_t* __restrict__ Gmm16,
-                              uint16_t* __restrict__ Gsm16, uint8_t* __restrict__ Gmm8, uint8_t* __restrict__ Gsm8) {
-  __shared__ uint8_t sval[64][128 + 2];
-  const int64_t m0 = (int64_t)blockIdx.x * 64;
-  const int64_t s0 = (int64_t)blockIdx.y * 128;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < 64 * 128; e += blockDim.x) {
-    const int mm = e >> 7, s = e & 127;
-    const int64_t mk = m0 + mm, smp = s0 + s;
-    uint8_t g = 0;
-    if (mk < m && smp < nn) {
-      const uint32_t f = (codes[mk * pitch + (smp >> 2)] >> (2 * (smp & 3))) & 3u;
-      g = (uint8_t)(f == 1u ? fill[mk] : field_geno(f));
+__device__ __forceinline__ void store_g(uint32_t copies, int form, uint16_t* __restrict__ o16, uint8_t* __restrict__ o8) {
+  uint32_t w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int a = (copies >> (4 * i)) & 3, b = (copies >> (4 * i + 2)) & 3;
+    w[i] = form ? g_f16(a) | ((uint32_t)g_f16(b) << 16) : g_bf16(a) | ((uint32_t)g_bf16(b) << 16);
+  }
+  uint4* o = reinterpret_cast<uint4*>(o16);
+  o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  if (form) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      w[i] = 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[i] |= (uint32_t)g_e4m3((copies >> (2 * (4 * i + e))) & 3) << (8 * e);
     }
-    sval[mm][s] = g;
-    Gmm16[mk * np + smp] = form ? g_f16(g) : g_bf16(g);
-    if (form) Gmm8[mk * np + smp] = g_e4m3(g);
+    *reinterpret_cast<uint4*>(o8) = make_uint4(w[0], w[1], w[2], w[3]);
   }
-  __syncthreads();
-  for (int e = tid; e < 64 * 128; e += blockDim.x) {
-    const int mm = e & 63, s = e >> 6;
-    const int g = sval[mm][s];
-    Gsm16[(s0 + s) * mg + m0 + mm] = form ? g_f16(g) : g_bf16(g);
-    if (form) Gsm8[(s0 + s) * mg + m0 + mm] = g_e4m3(g);
-  }
+}
+
+// Rows of markers: a thread takes one word (16 samples) of a row.
+__global__ void __launch_bounds__(kThreads)
+gbuild_mm_kernel(const uint8_t* __restrict__ codes, int64_t pitch, const int32_t* __restrict__ fill, int64_t m, int64_t nn,
+                 int64_t np, int form, uint16_t* __restrict__ G16, uint8_t* __restrict__ G8) {
+  const int64_t mk = blockIdx.x, s0 = 16 * ((int64_t)blockIdx.y * kThreads + threadIdx.x);
+  if (s0 >= np) return;
+  uint32_t x = 0;
+  if (mk < m && s0 < nn)
+    x = pack_copies(*reinterpret_cast<const uint32_t*>(codes + mk * pitch + s0 / 4), fill[mk], valid_fields(nn - s0));
+  store_g(x, form, G16 + mk * np + s0, form ? G8 + mk * np + s0 : nullptr);
+}
+
+// Rows of samples: a thread turns 16 markers x 16 samples; a warp reads 32 bytes of a marker row (8 words) and writes
+// 64 markers of a sample (128 bytes).
+__global__ void __launch_bounds__(kThreads)
+gbuild_sm_kernel(const uint8_t* __restrict__ codes, int64_t pitch, const int32_t* __restrict__ fill, int64_t m, int64_t nn,
+                 int64_t mg, int form, uint16_t* __restrict__ G16, uint8_t* __restrict__ G8) {
+  // block = 128 samples x 512 markers
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t k0 = (int64_t)blockIdx.x * 512 + 64 * warp + 16 * (lane & 3), s0 = (int64_t)blockIdx.y * 128 + 16 * (lane >> 2);
+  if (k0 >= mg) return;
+  const int64_t left = nn - s0;
+  const uint32_t valid = valid_fields(left);
+  uint32_t w[16];
+#pragma unroll
+  for (int p = 0; p < 16; ++p)
+    // pitch is a multiple of 16, so a word that starts inside a row ends there
+    w[p] = k0 + p < m && left > 0
+               ? pack_copies(*reinterpret_cast<const uint32_t*>(codes + (k0 + p) * pitch + s0 / 4), fill[k0 + p], valid)
+               : 0u;
+  transpose_fields(w);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) store_g(w[i], form, G16 + (s0 + i) * mg + k0, form ? G8 + (s0 + i) * mg + k0 : nullptr);
 }
 
 void launch_gbuild(const uint8_t* codes, int64_t pitch, const int32_t* fill, int64_t m, int64_t nn,
                    int64_t mg, int64_t np, int form, void* Gmm16, void* Gsm16, void* Gmm8, void* Gsm8,
                    cudaStream_t s) {
-  dim3 grid((unsigned)(mg / 64), (unsigned)(np / 128));
-  gbuild_kernel<<<grid, kThreads, 0, s>>>(codes, pitch, fill, m, nn, mg, np, form, static_cast<uint16_t*>(Gmm16),
-                                          static_cast<uint16_t*>(Gsm16), static_cast<uint8_t*>(Gmm8),
-                                          static_cast<uint8_t*>(Gsm8));
+  const int64_t words = np / 16;
+  gbuild_mm_kernel<<<dim3((unsigned)mg, (unsigned)((words + kThreads - 1) / kThreads)), kThreads, 0, s>>>(
+      codes, pitch, fill, m, nn, np, form, static_cast<uint16_t*>(Gmm16), static_cast<uint8_t*>(Gmm8));
+  gbuild_sm_kernel<<<dim3((unsigned)((mg + 511) / 512), (unsigned)(np / 128)), kThreads, 0, s>>>(
+      codes, pitch, fill, m, nn, mg, form, static_cast<uint16_t*>(Gsm16), static_cast<uint8_t*>(Gsm8));
 }
 
 // The same genotype values in two bits for the products of few columns (tc_packed_kernel), in both
