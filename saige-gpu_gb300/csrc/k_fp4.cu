@@ -26,7 +26,7 @@
 //
 // What runs here: the subset-exact products of the drop-ins that return FP32 (few columns, so G's
 // stream from HBM bounds them: half a byte a genotype and product against two).  Measured at N = 100k,
-// M = 150k, both products and the kernels around them: 15.4 against 62.2 ms for one AI score (4.0x); the
+// M = 150k, both products and the kernels around them: 15.0 against 62.2 ms for one AI score (4.1x); the
 // 32-column GEMM 1.08 ms, 7.5 GB at 1.02 of the copy rate.
 //
 // CTA pairs (cta_group::2): a pair computes 256 rows x CT vector columns (7 CT accumulator columns,
