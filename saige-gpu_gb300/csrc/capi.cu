@@ -2586,10 +2586,13 @@ static int step_finish(sg_ctx* c, int64_t* n_finished) {
   e.inflight = false;
   SG_TRY(sync(c));
   const auto th0 = std::chrono::steady_clock::now();
-  if (tc_mode(c->mv_mode) && *e.h_err != 0) {  // a bounded wait gave up: read and clear the device's flag
+  if (tc_mode(c->mv_mode) && *e.h_err != 0) {
+    // a bounded wait gave up.  The step's own copy of the flag decides: the device's is one per process, and another
+    // context's check may have read and cleared it since
     *e.h_err = 0;
-    const cudaError_t err = tc_check_error(c->stream);
-    if (err != cudaSuccess) return set_err(c, SG_ERR_CUDA, "tcgen05 GRM.V: %s", cudaGetErrorString(err));
+    cudaError_t err = tc_check_error(c->stream);
+    if (err == cudaSuccess) err = cudaErrorLaunchTimeout;
+    return set_err(c, SG_ERR_CUDA, "tcgen05 GRM.V: %s", cudaGetErrorString(err));
   }
   const int64_t ncols = e.inflight_ncols, occupied = e.inflight_occupied, hi = e.inflight_hi;
   {

@@ -1,9 +1,11 @@
 """Failure detection without faulting the GPU: bounded device waits, host-side refusals and
 per-request failures that leave the other requests running."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from saigegpu import GRM_FP32_SIMT, MV_FP32_SIMT, Context, SaigeGpuError, prep, serve, synth
+from saigegpu import GRM_FP32_SIMT, MV_FP32_SIMT, MV_SUBSET_EXACT, Context, SaigeGpuError, prep, serve, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -72,3 +74,41 @@ def test_failing_and_cancelled_fits_do_not_stop_the_others():
         assert str(by[ids[1]].error) == "cancelled"
         for i in (ids[0], ids[3]):
             assert by[i].error is None and by[i].result["converged"]
+
+
+@pytest.mark.parametrize("cleared", [False, True])
+def test_a_step_whose_wait_ran_out_fails(cleared):
+    """The flag the tcgen05 kernels set when a wait runs out, set from the host before a step: the step fails, also
+    when the process-wide flag has been read and cleared (as another context's check does) before it is finished."""
+    n, m = 256, 300
+    bed, _ = synth.synth_bed(6, n, m, 0.0)
+    V = np.random.default_rng(0).standard_normal((n, 2))
+    cuda = C.CDLL("libcuda.so.1")
+    with Context(0) as ctx:
+        flag = ctx._L._ZN2sg16tc_error_addressEv
+        flag.restype = C.c_void_p
+        address = C.c_uint64(flag())
+        assert address.value
+
+        def put(v):
+            assert cuda.cuMemcpyHtoD_v2(address, C.byref(C.c_int(v)), C.c_size_t(4)) == 0
+
+        ctx.setgeno(bed, n, m)
+        ctx.set_matvec_mode(MV_SUBSET_EXACT)
+        ctx.engine_reserve(32, 1)
+        ctx.engine_set_pheno(0, np.ones(n), np.array([1.0, 0.3]))
+        ids = ctx.engine_submit(0, 1, V)
+        put(3)
+        try:
+            ctx.engine_launch()
+            ctx.engine_wait()
+            if cleared:
+                put(0)
+            with pytest.raises(SaigeGpuError) as ei:
+                ctx.engine_finish()
+            assert ei.value.code == 2  # SG_ERR_CUDA
+        finally:
+            put(0)
+        for i in ids:
+            ctx.engine_cancel(i)
+        np.testing.assert_allclose(ctx.grm_matmul(V), ctx.grm_matmul(V), rtol=0, atol=0)  # still usable
