@@ -34,6 +34,7 @@ struct Req {
   int maxiter = 0;
   double tol = 0.0;
   bool probe = false;
+  bool may_stop = false;  // may converge at init: its right-hand side is small (or only on the device), or maxiter is 0
   uint64_t seed = 0;
   int64_t run = 0;
   double* b = nullptr;        // right-hand side in a pinned slab until admission copies it up
@@ -183,6 +184,7 @@ struct Engine {
   double* spart = nullptr;        // column partials: cap_cols x max(blocks over np, over mg)
   float* smax = nullptr;          // FP16 / E4M3 form: column block maxima, as spart
   float* sscale = nullptr;        //   and the columns' power-of-two scales s1, s2 (2 x cap_cols)
+  bool may_stop = false;          // a column admitted since the last step may have converged at init
   bool list_up = false;           // the step's active columns are on the device
   std::vector<int32_t> last_list;  // what d_gcols holds
   double* pap = nullptr;          // block partials of p'Ap: cap_cols x nblk
@@ -2026,6 +2028,16 @@ extern "C" int sg_engine_set_pheno(sg_ctx* c, int64_t slot, const double* w, con
   return SG_OK;
 }
 
+// Whether sum v^2 > limit; reads no further than it takes to see that.
+static bool norm2_exceeds(const double* v, int64_t n, double limit) {
+  double s = 0.0;
+  for (int64_t i = 0; i < n; ++i) {
+    s += v[i] * v[i];
+    if (s > limit) return true;
+  }
+  return false;
+}
+
 static int engine_submit_common(sg_ctx* c, int64_t slot, int kind, const double* B, bool probe,
                                 uint64_t seed, int64_t run0, int64_t k, int maxiter, double tol,
                                 int64_t* ids) {
@@ -2044,6 +2056,7 @@ static int engine_submit_common(sg_ctx* c, int64_t slot, int kind, const double*
     r.maxiter = maxiter;
     r.tol = tol;
     r.probe = probe;
+    r.may_stop = kind == 0 && (maxiter <= 0 || (probe ? !(tol < 1.0) : !norm2_exceeds(B + j * c->nn, c->nn, tol)));
     r.seed = seed;
     r.run = run0 + j;
     if (!probe) {
@@ -2092,6 +2105,7 @@ extern "C" int sg_engine_submit_chained(sg_ctx* c, int64_t slot, const int64_t* 
     r.kind = 0;
     r.maxiter = maxiter;
     r.tol = tol;
+    r.may_stop = true;
     r.src = src_ids[j];
     // a slab for the source's result, should the source be fetched before this one is admitted
     if (!slab_get(c, r)) return set_err(c, SG_ERR_NOMEM, "no pinned host memory for a right-hand side");
@@ -2288,6 +2302,7 @@ static int engine_admit(sg_ctx* c) {
       // is skipped by the vector kernels and retired when the step finishes)
       e.h_st[col] = s;
       e.h_st[col].active = 1;
+      e.may_stop = e.may_stop || r.may_stop;
       e.col_req[col] = id;
       r.col = col;
       r.state = 1;
@@ -2548,6 +2563,7 @@ static int step_launch(sg_ctx* c) {
   // back); the GRM.V compaction and the vector kernels work on this list only
   e.nact = 0;
   e.list_up = false;
+  e.may_stop = false;
   for (int64_t col = 0; col < e.hi_col; ++col)
     if (e.h_st[col].active) e.h_gcols[e.nact++] = (int32_t)col;
   // the split-BF16 engine compacts the active columns itself; the others cover [0, hi_col) padded
@@ -2674,6 +2690,44 @@ static int engine_step(sg_ctx* c, int64_t* n_finished) {
   return step_finish(c, n_finished);
 }
 
+// Columns that converged at init (r'r <= tol, or no iteration allowed) retire without a step, iter = 0 and x = 0.  Reads
+// the fresh states back, which waits for the device: called only where a right-hand side says it may be one of those.
+static int engine_retire_immediate(sg_ctx* c, int64_t* n_finished) {
+  Engine& e = c->eng;
+  if (!e.may_stop) return SG_OK;
+  e.may_stop = false;
+  if (e.hi_col == 0) return SG_OK;
+  SG_CUDA(c, d2h(c, e.h_st.data(), e.d_st, e.hi_col * sizeof(ColState), c->stream));
+  SG_TRY(sync(c));
+  for (int64_t col = 0; col < e.hi_col; ++col) {
+    const int64_t id = e.col_req[col];
+    if (id < 0) continue;
+    ColState& s = e.h_st[col];
+    if (s.kind != 0 || s.active || !s.just_done) continue;
+    auto it = e.reqs.find(id);
+    if (it != e.reqs.end()) {
+      it->second.iters = 0;
+      it->second.state = 2;
+      it->second.col = e.hold ? col : -1;  // X[col] was zeroed at admission
+      if (!e.hold) it->second.x.assign(c->nn, 0.0);
+      e.finished.push_back(id);
+    }
+    e.n_active -= 1;
+    e.retired += 1;
+    *n_finished += 1;
+    if (e.hold && it != e.reqs.end()) {
+      s.kind = -2;
+      s.just_done = 0;
+      stage_state(e, col, s);
+    } else {
+      SG_TRY(release_col(c, col));
+    }
+  }
+  while (e.hi_col > 0 && e.col_req[e.hi_col - 1] == -1) --e.hi_col;
+  SG_TRY(flush_states(c, false));
+  return sync(c);
+}
+
 extern "C" int sg_engine_run(sg_ctx* c, int64_t max_steps, int64_t* n_finished) {
   NEED_OPERATOR(c);
   Engine& e = c->eng;
@@ -2688,8 +2742,8 @@ extern "C" int sg_engine_run(sg_ctx* c, int64_t max_steps, int64_t* n_finished) 
   }
   for (int64_t s = 0; s < max_steps; ++s) {
     SG_TRY(engine_admit(c));
-    // columns that converged at init (iter = 0, x = 0) retire when this step finishes: reading the fresh
-    // states back first would cost every call a round trip
+    SG_TRY(engine_retire_immediate(c, &fin));
+    if (fin > 0) break;
     if (e.n_active == 0) {
       if (!e.queue.empty())
         return set_err(c, SG_ERR_STATE,

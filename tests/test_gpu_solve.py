@@ -156,3 +156,43 @@ def test_masked_phenotype_equals_subset_system(cohort):
     exact = np.linalg.solve(Ss, b[S])
     assert np.linalg.norm(x[S] - exact) / np.linalg.norm(exact) < 1e-5
     assert not x[mask == 0].any()
+
+
+def test_right_hand_sides_that_converge_at_init_take_no_step(gpu_ctx):
+    """r'r <= tol at the start (a zero or small right-hand side) or no iteration allowed: x = 0, iter = 0, no GRM product;
+    beside a column that iterates, that column's own result."""
+    from saigegpu import MV_FP32_SIMT, MV_SUBSET_EXACT
+    n, m = 300, 500
+    bed, _ = synth.synth_bed(71, n, m, 0.01)
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    w, tau = np.ones(n, np.float32), np.array([0.6, 0.4], np.float32)
+    b = np.random.default_rng(0).standard_normal(n).astype(np.float32)
+    ctx.set_matvec_mode(MV_SUBSET_EXACT)
+    try:
+        alone = ctx.getSigma_X(w, tau, b[:, None])
+        steps = ctx.engine_stats()["steps"]
+        for v, maxiter, tol in ((0 * b, 500, 1e-5), (b, 0, 1e-5), (b, 500, 1e6), (1e-4 * b, 500, 1e-5)):
+            x, it = ctx.getPCG1ofSigmaAndVector(w, tau, v.astype(np.float32), maxiter, tol, return_iters=True)
+            assert it == 0 and not x.any()
+        assert not ctx.getSigma_X(w, tau, np.zeros((n, 3), np.float32)).any()
+        assert ctx.engine_stats()["steps"] == steps
+        X = ctx.getSigma_X(w, tau, np.column_stack([0 * b, b, 0 * b]))
+        np.testing.assert_array_equal(X[:, 1], alone[:, 0])
+        assert not X[:, [0, 2]].any()
+        # results held on the device, and a chained solve of one of them
+        ctx.engine_set_pheno(0, np.ones(n), np.array([0.6, 0.4]))
+        ctx.engine_hold_results(True)
+        steps = ctx.engine_stats()["steps"]
+        i = int(ctx.engine_submit(0, 0, np.zeros((n, 1)))[0])
+        ctx.engine_run()
+        j = int(ctx.engine_submit_chained(0, [i])[0])
+        ctx.engine_run()
+        for k in (j, i):
+            x, it = ctx.engine_fetch(k)
+            assert it == 0 and not x.any()
+        assert ctx.engine_stats()["steps"] == steps
+    finally:
+        ctx.engine_hold_results(False)
+        ctx.set_matvec_mode(MV_FP32_SIMT)
