@@ -338,6 +338,14 @@ static int set_err(sg_ctx* c, int code, const char* fmt, ...) {
 
 static bool release_spares(sg_ctx* c);
 
+// While it lives, allocations are of what only saves time (the spare genotype copies, staging buffers of copies that can
+// go without): nothing makes room for them.
+struct SpareScope {
+  sg_ctx* c;
+  explicit SpareScope(sg_ctx* ctx) : c(ctx) { c->spare_alloc = true; }
+  ~SpareScope() { c->spare_alloc = false; }
+};
+
 static int dev_alloc(sg_ctx* c, void** p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) bytes = 16;
@@ -873,6 +881,7 @@ static int bed_upload(sg_ctx* c, const uint8_t* body, int64_t nb, int64_t m, int
                       int64_t raw_pitch) {
   if (m == 0) return SG_OK;
   const int64_t rows = std::min(m, std::max<int64_t>(1, kBedStage / nb));
+  const SpareScope spare(c);
   uint8_t* flat = nullptr;
   const std::string err = c->err;
   if (dev_alloc_t(c, &flat, (size_t)(rows * nb + 16)) != SG_OK) {
@@ -1039,6 +1048,7 @@ extern "C" int sg_get_packed_geno(sg_ctx* c, uint8_t* out) {
   const int64_t nb = (c->nn + 3) / 4;
   if (c->m_qc == 0) return SG_OK;
   const int64_t rows = std::min(c->m_qc, std::max<int64_t>(1, kBedStage / nb));
+  const SpareScope spare(c);
   uint8_t* flat = nullptr;
   const std::string err = c->err;
   if (nb == c->pitch || dev_alloc_t(c, &flat, (size_t)(rows * nb + 16)) != SG_OK) {
@@ -1348,13 +1358,6 @@ static bool release_spares(sg_ctx* c) {
   c->gp_refused = c->g4_refused = c->gk_refused = true;
   return true;
 }
-
-// While it lives, allocations are of such copies.
-struct SpareScope {
-  sg_ctx* c;
-  explicit SpareScope(sg_ctx* ctx) : c(ctx) { c->spare_alloc = true; }
-  ~SpareScope() { c->spare_alloc = false; }
-};
 
 // Scratch of the FP4 products over up to mg markers (a multiple of 128).
 static int fp4_scratch(sg_ctx* c, int64_t mg) {

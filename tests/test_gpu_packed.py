@@ -67,3 +67,30 @@ def test_gives_way_to_other_memory():
         np.testing.assert_array_equal(o, a)
     assert c[3] == used1 - packed
     assert d[2] == used1 and d[3] == used2 - packed
+
+
+def test_a_read_back_leaves_the_copies(gpu_ctx):
+    """packed_geno()'s staging buffer only saves time: under a budget with no room for it the two-bit and E2M1 copies
+    stay, and the rows are copied without it."""
+    n, m = 500, 900
+    bed, _ = synth.synth_bed(9, n, m, 0.02)
+    b = np.random.default_rng(1).standard_normal(n).astype(np.float32)
+
+    def run(budget):
+        with Context(0, budget) as ctx:
+            ctx.setgeno(bed, n, m)
+            ctx.set_matvec_mode(MV_SUBSET_EXACT)
+            ctx.engine_reserve(128, 1)
+            y = ctx.grm_matmul(b), ctx.getCrossprodMatAndKin(b)
+            used = ctx.bytes_in_use()
+            packed = ctx.packed_geno()
+            assert ctx.bytes_in_use() == used
+            return used, packed, y, (ctx.grm_matmul(b), ctx.getCrossprodMatAndKin(b))
+
+    used, packed, y, again = run(0)
+    tight = run(used)
+    assert tight[0] == used
+    np.testing.assert_array_equal(tight[1], packed)
+    for got in (again, tight[2], tight[3]):
+        for a, o in zip(got, y):
+            np.testing.assert_array_equal(a, o)
