@@ -336,7 +336,7 @@ static int set_err(sg_ctx* c, int code, const char* fmt, ...) {
     if (r_ != SG_OK) return r_; \
   } while (0)
 
-static bool release_spares(sg_ctx* c);
+static bool release_spares(sg_ctx* c, size_t bytes);
 
 // While it lives, allocations are of what only saves time (the spare genotype copies, staging buffers of copies that can
 // go without): nothing makes room for them.
@@ -351,7 +351,7 @@ static int dev_alloc(sg_ctx* c, void** p, size_t bytes) {
   if (bytes == 0) bytes = 16;
   auto over = [&] { return c->budget && c->in_use + bytes > c->budget; };
   cudaError_t e = over() ? cudaSuccess : cudaMalloc(p, bytes);
-  if ((over() || e != cudaSuccess) && release_spares(c)) {
+  if ((over() || e != cudaSuccess) && release_spares(c, bytes)) {
     cudaGetLastError();
     e = over() ? cudaSuccess : cudaMalloc(p, bytes);
   }
@@ -1346,10 +1346,22 @@ static void fp4_free(sg_ctx* c) {
   w = Fp4Scratch{};
 }
 
-// Gives back the genotype copies that only save time (two-bit, E2M1), for an allocation that has to succeed.  Their
-// products run as the others from then on.
-static bool release_spares(sg_ctx* c) {
-  if (c->spare_alloc || (!c->d_Gp && !c->d_G4 && !c->d_Gk && !c->eng.f4.Vq)) return false;
+// Gives back the genotype copies that only save time (two-bit, E2M1), for an allocation of ``bytes`` that has to
+// succeed, if it then can.  Their products run as the others from then on.
+static bool release_spares(sg_ctx* c, size_t bytes) {
+  if (c->spare_alloc) return false;
+  const Fp4Scratch& w = c->eng.f4;
+  size_t held = 0;
+  for (const void* p : {c->d_Gp, c->d_G4, c->d_Gk, (void*)c->d_gk_slot, (void*)c->d_gk_p2d, (void*)c->d_gk_dp,
+                        (void*)c->d_gk_p2, w.Vq, w.Tq, (void*)w.T, (void*)w.U, (void*)w.part, (void*)w.qsum,
+                        (void*)w.pmax, (void*)w.mean, (void*)w.descale1, (void*)w.descale2}) {
+    const auto it = c->allocs.find(const_cast<void*>(p));
+    if (it != c->allocs.end()) held += it->second;
+  }
+  size_t unused = 0, total = 0;
+  if (held == 0 || (c->budget && c->in_use - held + bytes > c->budget) ||
+      cudaMemGetInfo(&unused, &total) != cudaSuccess || unused + held < bytes)
+    return false;
   dev_free(c, c->d_Gp);
   dev_free(c, c->d_G4);
   c->d_Gp = c->d_G4 = nullptr;

@@ -3,7 +3,7 @@ on CTA pairs: the same products in the same order, so the same bits."""
 import numpy as np
 import pytest
 
-from saigegpu import MV_FP32_SIMT, MV_SUBSET_EXACT, TC_SUBSET_PAIR, Context, synth
+from saigegpu import MV_FP32_SIMT, MV_SUBSET_EXACT, TC_SUBSET_PAIR, Context, SaigeGpuError, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +94,23 @@ def test_a_read_back_leaves_the_copies(gpu_ctx):
     for got in (again, tight[2], tight[3]):
         for a, o in zip(got, y):
             np.testing.assert_array_equal(a, o)
+
+
+def test_a_request_that_cannot_fit_leaves_the_copies():
+    """An allocation beyond the budget even without the copies is refused and takes nothing from them."""
+    n, m = 500, 900
+    bed, _ = synth.synth_bed(9, n, m, 0.02)
+    b = np.random.default_rng(1).standard_normal(n).astype(np.float32)
+    with Context(0, 1 << 30) as ctx:
+        ctx.setgeno(bed, n, m)
+        ctx.set_matvec_mode(MV_SUBSET_EXACT)
+        ctx.engine_reserve(128, 1)
+        y, z = ctx.grm_matmul(b), ctx.getCrossprodMatAndKin(b)
+        used = ctx.bytes_in_use()
+        with pytest.raises(SaigeGpuError) as ei:
+            ctx.synth_bed(1, 1 << 20, 1 << 14, 0.0)  # 4 GB
+        assert ei.value.code == 3  # SG_ERR_NOMEM
+        assert ctx.bytes_in_use() == used
+        np.testing.assert_array_equal(ctx.grm_matmul(b), y)
+        np.testing.assert_array_equal(ctx.getCrossprodMatAndKin(b), z)
+        assert ctx.bytes_in_use() == used
