@@ -1425,10 +1425,8 @@ static bool fp4_ready(sg_ctx* c) {
   const std::string err = c->err;
   if (all() != SG_OK) {
     fp4_free(c);
-    if (build) {
-      dev_free(c, c->d_G4);
-      c->d_G4 = nullptr;
-    }
+    dev_free(c, c->d_G4);  // built earlier or not: without the scratch it serves nothing
+    c->d_G4 = nullptr;
     c->g4_refused = true;
     c->err = err;
     return false;

@@ -168,3 +168,34 @@ def test_drop_ins_on_a_resident_grm(gpu_ctx, mode, n, m):
         assert np.abs(y - want).max() < (4 * 2.0 ** -17 if mode == MV_BF16X3_TC else TOL) * np.abs(want).max()
     finally:
         ctx.set_matvec_mode(MV_FP32_SIMT)
+
+
+def test_refused_scratch_gives_the_matrix_back():
+    """A larger engine whose FP4 scratch no longer fits the budget: the E2M1 matrix, built for the smaller one, goes too
+    and the drop-ins run on the BF16 products."""
+    from saigegpu import Context
+    n, m = 500, 900
+    bed, _ = synth.synth_bed(9, n, m, 0.02)
+    b = np.random.default_rng(1).standard_normal(n).astype(np.float32)
+
+    def run(budget):
+        with Context(0, budget) as ctx:
+            ctx.setgeno(bed, n, m)
+            ctx.set_matvec_mode(MV_SUBSET_EXACT)
+            used, out = [], []
+            for cols in (128, 256):
+                ctx.engine_reserve(cols, 1)
+                ctx.grm_matmul(b)  # the BF16 products' scratch
+                used.append(ctx.bytes_in_use())
+                out.append(ctx.getCrossprodMatAndKin(b))
+                used.append(ctx.bytes_in_use())
+            assert not budget or np.array_equal(out[1], ctx.grm_matmul(b).astype(np.float32))
+            return used, out
+
+    used, out = run(0)
+    np.testing.assert_array_equal(out[0], out[1])
+    tight = run(used[3] - 16)
+    assert tight[0][:2] == used[:2]
+    np.testing.assert_array_equal(tight[1][0], out[0])
+    matrix = 12288 * (8 * 3 + 4 * 5)  # row blocks of 128 (markers, samples) x stages of 192 (samples, markers)
+    assert tight[0][2] == used[2] and tight[0][3] == used[2] - matrix
