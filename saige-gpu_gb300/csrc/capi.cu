@@ -277,6 +277,7 @@ struct sg_ctx {
   void* d_Gp = nullptr;
   bool gp_refused = false;  // no memory for it: those products read d_G
   bool spare_alloc = false;  // what is being allocated only saves time, so nothing makes room for it
+  uint64_t refused_at = 0;   // in_use when memory for one of these copies was last refused or taken back
   // the same values in E2M1 for the FP32 drop-ins' products (k_fp4.cu), built at the first of them
   void* d_G4 = nullptr;
   bool g4_refused = false;  // no memory for it: those products run as the others
@@ -351,7 +352,8 @@ static int dev_alloc(sg_ctx* c, void** p, size_t bytes) {
   if (bytes == 0) bytes = 16;
   auto over = [&] { return c->budget && c->in_use + bytes > c->budget; };
   cudaError_t e = over() ? cudaSuccess : cudaMalloc(p, bytes);
-  if ((over() || e != cudaSuccess) && release_spares(c, bytes)) {
+  const bool released = (over() || e != cudaSuccess) && release_spares(c, bytes);
+  if (released) {
     cudaGetLastError();
     e = over() ? cudaSuccess : cudaMalloc(p, bytes);
   }
@@ -365,6 +367,7 @@ static int dev_alloc(sg_ctx* c, void** p, size_t bytes) {
   }
   c->allocs[*p] = bytes;
   c->in_use += bytes;
+  if (released) c->refused_at = c->in_use;
   return SG_OK;
 }
 
@@ -1347,7 +1350,7 @@ static void fp4_free(sg_ctx* c) {
 }
 
 // Gives back the genotype copies that only save time (two-bit, E2M1), for an allocation of ``bytes`` that has to
-// succeed, if it then can.  Their products run as the others from then on.
+// succeed, if it then can.  Their products run as the others while that memory is in use.
 static bool release_spares(sg_ctx* c, size_t bytes) {
   if (c->spare_alloc) return false;
   const Fp4Scratch& w = c->eng.f4;
@@ -1369,6 +1372,17 @@ static bool release_spares(sg_ctx* c, size_t bytes) {
   fp4_free(c);
   c->gp_refused = c->g4_refused = c->gk_refused = true;
   return true;
+}
+
+// A copy was refused (``flag``): its products run as the others until this context uses less memory than it did then.
+static void spare_refuse(sg_ctx* c, bool& flag, const std::string& err) {
+  flag = true;
+  c->refused_at = c->in_use;
+  c->err = err;
+}
+static bool spare_refused(sg_ctx* c, const bool& flag) {
+  if (flag && c->in_use < c->refused_at) c->gp_refused = c->g4_refused = c->gk_refused = false;
+  return flag;
 }
 
 // Scratch of the FP4 products over up to mg markers (a multiple of 128).
@@ -1394,13 +1408,12 @@ static int fp4_scratch(sg_ctx* c, int64_t mg) {
 // memory (or budget) for it.
 static bool gpack_ready(sg_ctx* c) {
   if (c->d_Gp) return true;
-  if (c->gp_refused) return false;
+  if (spare_refused(c, c->gp_refused)) return false;
   const SpareScope spare(c);
   const int64_t each = gpack_bytes(c->mg, c->eng.np);
   const std::string err = c->err;
   if (dev_alloc(c, &c->d_Gp, (size_t)(2 * each)) != SG_OK) {
-    c->gp_refused = true;
-    c->err = err;
+    spare_refuse(c, c->gp_refused, err);
     return false;
   }
   uint8_t* g = static_cast<uint8_t*>(c->d_Gp);
@@ -1414,7 +1427,7 @@ static bool gpack_ready(sg_ctx* c) {
 static bool fp4_ready(sg_ctx* c) {
   Engine& e = c->eng;
   if (c->d_G4 && e.f4.T && e.f4.mg >= c->mg) return true;
-  if (c->g4_refused) return false;
+  if (spare_refused(c, c->g4_refused)) return false;
   const SpareScope spare(c);
   const int64_t mm = fp4_matrix_bytes(c->mg, c->nn);
   const bool build = !c->d_G4;
@@ -1427,8 +1440,7 @@ static bool fp4_ready(sg_ctx* c) {
     fp4_free(c);
     dev_free(c, c->d_G4);  // built earlier or not: without the scratch it serves nothing
     c->d_G4 = nullptr;
-    c->g4_refused = true;
-    c->err = err;
+    spare_refuse(c, c->g4_refused, err);
     return false;
   }
   if (build) {
@@ -1437,7 +1449,7 @@ static bool fp4_ready(sg_ctx* c) {
       fp4_free(c);
       dev_free(c, c->d_G4);
       c->d_G4 = nullptr;
-      c->g4_refused = true;
+      spare_refuse(c, c->g4_refused, err);
       return false;
     }
     c->launches += 2;
@@ -1480,15 +1492,14 @@ static int fp4_cohort_build(sg_ctx* c) {
 }
 
 static bool fp4_cohort_ready(sg_ctx* c) {
-  if (c->gk_refused) return false;
+  if (spare_refused(c, c->gk_refused)) return false;
   const SpareScope spare(c);
   const std::string err = c->err;
   const int64_t mg = round_up(c->m_qc, kRowTile);
   if ((!c->d_Gk && fp4_cohort_build(c) != SG_OK) || fp4_scratch(c, mg) != SG_OK) {
     fp4_free(c);
     free_gk(c);
-    c->gk_refused = true;
-    c->err = err;
+    spare_refuse(c, c->gk_refused, err);
     return false;
   }
   return true;

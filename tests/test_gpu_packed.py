@@ -114,3 +114,32 @@ def test_a_request_that_cannot_fit_leaves_the_copies():
         np.testing.assert_array_equal(ctx.grm_matmul(b), y)
         np.testing.assert_array_equal(ctx.getCrossprodMatAndKin(b), z)
         assert ctx.bytes_in_use() == used
+
+
+def test_copies_come_back_with_the_memory():
+    """What made the copies give way is freed: the next products build them again, and give the same bits."""
+    n, m, big = 500, 900, 2 << 20
+    bed, _ = synth.synth_bed(9, n, m, 0.02)
+    b = np.random.default_rng(1).standard_normal(n).astype(np.float32)
+
+    def run(budget):
+        with Context(0, budget) as ctx:
+            ctx.setgeno(bed, n, m)
+            ctx.set_matvec_mode(MV_SUBSET_EXACT)
+            ctx.engine_reserve(128, 1)
+            used, out = [], []
+            for size in (16, big, 16):
+                ctx.synth_bed(1, 4, size, 0.0)  # ``size`` bytes that have to be there
+                out.append((ctx.grm_matmul(b), ctx.getCrossprodMatAndKin(b)))
+                used.append(ctx.bytes_in_use())
+            return used, out
+
+    used, out = run(0)
+    assert used[1] == used[0] + big - 16 and used[2] == used[0]
+    tight, got = run(used[0] + 1024)
+    assert tight[0] == used[0] and tight[1] < used[1] and tight[2] == used[2]
+    for i in range(3):
+        np.testing.assert_array_equal(got[i][0], out[0][0])
+    np.testing.assert_array_equal(got[1][1], got[1][0].astype(np.float32))  # the BF16 products meanwhile
+    for i in (0, 2):
+        np.testing.assert_array_equal(got[i][1], out[0][1])
