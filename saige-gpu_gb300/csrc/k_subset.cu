@@ -191,8 +191,8 @@ __global__ void __launch_bounds__(kThreads)
 gpack_mm_kernel(const uint8_t* __restrict__ codes, int64_t pitch, const int32_t* __restrict__ fill, int64_t m, int64_t nn,
                 int stages, uint4* __restrict__ out) {
   __shared__ uint4 sp[kPackPieces][kRowTile + 1];
-  const int ks0 = blockIdx.x * kPackStages;
-  const int64_t rb = blockIdx.y;
+  const int ks0 = blockIdx.y * kPackStages;
+  const int64_t rb = blockIdx.x;  // 65,536 row blocks and more are 8.4 million markers: grid.x has room
   for (int t = threadIdx.x; t < kRowTile * kPackPieces; t += kThreads) {
     const int row = t / kPackPieces, q = t % kPackPieces;
     const int64_t mk = rb * kRowTile + row, s0 = (int64_t)ks0 * kPackK + 64 * q;
@@ -255,7 +255,7 @@ int64_t gpack_bytes(int64_t mg, int64_t np) { return mg * np / 4; }
 void launch_gpack(const uint8_t* codes, int64_t pitch, const int32_t* fill, int64_t m, int64_t nn, int64_t mg,
                   int64_t np, void* Gmm, void* Gsm, cudaStream_t s) {
   const int sn = (int)(np / kPackK), sm = (int)(mg / kPackK);
-  gpack_mm_kernel<<<dim3((unsigned)((sn + kPackStages - 1) / kPackStages), (unsigned)(mg / kRowTile)), kThreads, 0, s>>>(
+  gpack_mm_kernel<<<dim3((unsigned)(mg / kRowTile), (unsigned)((sn + kPackStages - 1) / kPackStages)), kThreads, 0, s>>>(
       codes, pitch, fill, m, nn, sn, static_cast<uint4*>(Gmm));
   const int64_t rs = np / kRowTile;
   gpack_sm_kernel<<<dim3((unsigned)sm, (unsigned)((rs + 3) / 4)), kThreads, 0, s>>>(codes, pitch, fill, m, nn, sm, rs,

@@ -143,3 +143,28 @@ def test_copies_come_back_with_the_memory():
     np.testing.assert_array_equal(got[1][1], got[1][0].astype(np.float32))  # the BF16 products meanwhile
     for i in (0, 2):
         np.testing.assert_array_equal(got[i][1], out[0][1])
+
+
+def test_more_row_blocks_than_a_grid_has_rows(gpu_ctx):
+    """8.4 million markers of a few samples: 65,537 blocks of 128 rows."""
+    n, m = 8, 65536 * 128 + 5
+    ctx = gpu_ctx
+    body = np.random.default_rng(2).choice(np.array([0, 2, 3], np.uint8), (m, n))
+    body = body[:, 0::4] | (body[:, 1::4] << 2) | (body[:, 2::4] << 4) | (body[:, 3::4] << 6)
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(np.concatenate([np.array([0x6C, 0x1B, 0x01], np.uint8), body.ravel()]), n, m)
+    V = np.random.default_rng(3).standard_normal((n, 5))
+    try:
+        ctx.set_matvec_mode(MV_SUBSET_EXACT)
+        ctx.engine_reserve(32, 1)
+        out = []
+        for pair in (0, 1):
+            ctx.set_tc_option(TC_SUBSET_PAIR, pair)
+            out.append(ctx.grm_matmul(V))
+        np.testing.assert_array_equal(out[0], out[1])
+        assert np.abs(out[0]).max(0).min() > 0
+    finally:
+        ctx.set_tc_option(TC_SUBSET_PAIR, 2)
+        ctx.set_matvec_mode(MV_FP32_SIMT)
+        bed, _ = synth.synth_bed(9, 64, 90, 0.02)
+        ctx.setgeno(bed, 64, 90)  # the 4 GB of genotypes leave the shared context
