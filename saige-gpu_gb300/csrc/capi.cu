@@ -191,6 +191,7 @@ struct Engine {
   uint32_t* done = nullptr;       // per column, blocks of the direction kernel that have finished
   int* h_err = nullptr;           // pinned: the tcgen05 kernels' error flag as of the step's end
   int64_t fp32_cols = 0;          // > 0: a drop-in that returns FP32 runs, with steps of up to so many columns
+  bool fp32_used = false;         //   and a step of it took a form of its own (Fp32Form)
   Fp4Scratch f4;
   float* sdiag_part[kSetupStreams] = {};  // per-chunk partial sums of a subset's diagonal, per set-up stream
 
@@ -1516,7 +1517,11 @@ struct Fp32Scope {
     else outer = true;  // a drop-in inside another keeps the outer call's form
   }
   ~Fp32Scope() {
-    if (!outer) e.fp32_cols = 0;
+    if (outer) return;
+    e.fp32_cols = 0;
+    // products in these forms that the call left in slot 0's probe cache would answer an FP64 caller's probes
+    if (e.fp32_used && !e.pcache_key.empty()) e.pcache_key[0].clear();
+    e.fp32_used = false;
   }
   bool outer = false;
 };
@@ -2417,6 +2422,7 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
   *launched = ncols;
   const Fp32Form form = fp32_form(c);
   if (form != Fp32Form::kEngine) {
+    e.fp32_used = true;
     const int64_t nact = e.nact;
     *launched = nact;
     if (nact == 0) return SG_OK;

@@ -199,3 +199,25 @@ def test_refused_scratch_gives_the_matrix_back():
     np.testing.assert_array_equal(tight[1][0], out[0])
     matrix = 12288 * (8 * 3 + 4 * 5)  # row blocks of 128 (markers, samples) x stages of 192 (samples, markers)
     assert tight[0][2] == used[2] and tight[0][3] == used[2] - matrix
+
+
+@pytest.mark.parametrize("mode", [MV_SUBSET_EXACT, MV_FP32_SIMT])
+def test_drop_ins_leave_no_products_in_the_probe_cache(gpu_ctx, mode):
+    """K u of a drop-in's probes, computed in its own form, does not answer an FP64 caller of the engine."""
+    n, m, seed = 300, 500, 17
+    bed, _ = synth.synth_bed(61, n, m, 0.02)
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    ctx.grm_build(GRM_FP32_SIMT)
+    X = np.column_stack([np.ones(n), np.random.default_rng(0).standard_normal(n)]).astype(np.float32)
+    w, tau = np.ones(n, np.float32), np.array([0.6, 0.4], np.float32)
+    cov = np.linalg.inv(X.T @ X).astype(np.float32)
+    ctx.set_matvec_mode(mode)
+    try:
+        ctx.GetTrace_q(X, X, w, tau, cov, 10, seed=seed)
+        assert not any(ctx.engine_probe_cached(0, seed, r) for r in range(10))
+        ctx.getAIScore_q(X[:, 1], X, w, tau, X[:, 1], X, cov, 10, seed=seed)
+        assert not any(ctx.engine_probe_cached(0, seed, r) for r in range(10))
+    finally:
+        ctx.set_matvec_mode(MV_FP32_SIMT)
