@@ -77,14 +77,21 @@ __host__ __device__ __forceinline__ uint32_t digit_codes(int32_t q) {
   return w;
 }
 
-// Power of two that brings a column of magnitude at most ``bound`` into (2^23, 2^24] (exact), and 0
-// for a zero column.  The exponent is clamped where the scale or its inverse would leave FP32.
+// Exponent of the power of two that brings a column of magnitude at most ``bound`` into (2^23, 2^24] (exact), and 0
+// for a zero column; clamped where its inverse, the descale, would leave FP32 (it may be a subnormal).
 __device__ __forceinline__ int fixed_exponent(float bound) {
   if (!(bound > 0.0f)) return 0;
   int e = 0;
   frexpf(bound, &e);  // bound = f 2^e, f in [0.5, 1)
-  return min(max(24 - e, -120), 120);
+  return min(max(24 - e, -120), 148);
 }
+
+// x 2^e in two factors, each within FP32: 2^e alone leaves it for columns below 2^-103
+struct Scale {
+  float a, b;
+  __device__ __forceinline__ explicit Scale(int e) : a(ldexpf(1.0f, e / 2)), b(ldexpf(1.0f, e - e / 2)) {}
+  __device__ __forceinline__ float operator()(float x) const { return x * a * b; }
+};
 
 // Byte of vector column j's digit d, element k, in the digit operand of column tiles of CT columns
 // (S stages): tile, stage and CTA rank of the pair, then the CTA's rows (half h of 32 columns has
@@ -656,7 +663,8 @@ fp4_center_digits_kernel(const float* __restrict__ Pf, int64_t np, const int32_t
     }
   }
   __syncthreads();
-  const float mu = s_mu, sc = ldexpf(1.0f, s_e);
+  const float mu = s_mu;
+  const Scale sc(s_e);
   const int64_t k = (int64_t)blockIdx.x * kQChunk + 8 * threadIdx.x;
   int32_t q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (col >= 0 && k < np) {
@@ -667,8 +675,8 @@ fp4_center_digits_kernel(const float* __restrict__ Pf, int64_t np, const int32_t
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const double2 w = wv[i];
-      if (w.x != 0.0) q[2 * i] = __float2int_rn((v[2 * i] - mu) * sc);
-      if (w.y != 0.0) q[2 * i + 1] = __float2int_rn((v[2 * i + 1] - mu) * sc);
+      if (w.x != 0.0) q[2 * i] = __float2int_rn(sc(v[2 * i] - mu));
+      if (w.y != 0.0) q[2 * i + 1] = __float2int_rn(sc(v[2 * i + 1] - mu));
     }
   }
   if (k < (int64_t)dt.stages * kStageK) store_digits(out, dt, j, k, q);
@@ -779,7 +787,8 @@ fp4_scale_digits_kernel(const float* __restrict__ T, int64_t mg, const int32_t* 
   const int e = fixed_exponent(shm[0]);
   if (blockIdx.x == 0 && threadIdx.x == 0)
     descale[j] = shm[0] < 3.0e38f ? ldexpf(1.0f, -e) : __int_as_float(0x7fc00000);
-  const float sc = ldexpf(1.0f, e), inv = ldexpf(1.0f, -e);
+  const Scale sc(e);
+  const float inv = ldexpf(1.0f, -e);
   const int64_t k = (int64_t)blockIdx.x * kQChunk + 8 * threadIdx.x;
   double cf = 0.0;
   if (k < (int64_t)dt.stages * kStageK) {
@@ -794,7 +803,7 @@ fp4_scale_digits_kernel(const float* __restrict__ T, int64_t mg, const int32_t* 
         const double pp[4] = {p01.x, p01.y, p23.x, p23.y};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int32_t qi = __float2int_rn(x[i] * sc);
+          const int32_t qi = __float2int_rn(sc(x[i]));
           q[4 * h + i] = qi;
           // |q| <= 2^24 is exact in FP32; a value that is not finite stays so in the sum
           cf = fma(pp[i], (double)(isfinite(x[i]) ? (float)qi * inv : x[i]), cf);
@@ -844,12 +853,13 @@ fp4_finalize_kernel(const float* __restrict__ U, int64_t np, int64_t nn, const i
       if (w.y != 0.0) live |= 2u << (2 * i);
     }
   }
-  const float inv = descale[j], sc = 1.0f / inv;  // powers of two
+  const float inv = descale[j];  // a power of two, or NaN
+  const Scale sc(inv > 0.0f ? -ilogbf(inv) : 0);
   for (int f0 = 0; f0 < sl.nflip; f0 += kFinF) {
     const int fn = sl.nflip - f0 < kFinF ? sl.nflip - f0 : kFinF;
     __syncthreads();
     for (int q = threadIdx.x; q < fn; q += kQThreads)  // T' as GEMM 2 multiplied it
-      tf[q] = sl.dfill[f0 + q] * (rintf(T[j * mg + sl.flips[f0 + q]] * sc) * inv);
+      tf[q] = sl.dfill[f0 + q] * (rintf(sc(T[j * mg + sl.flips[f0 + q]])) * inv);
     __syncthreads();
     const int w0 = f0 / 32, wn = (fn + 31) / 32;
     for (int i = 0; i < 8; ++i) {

@@ -221,3 +221,24 @@ def test_drop_ins_leave_no_products_in_the_probe_cache(gpu_ctx, mode):
         assert not any(ctx.engine_probe_cached(0, seed, r) for r in range(10))
     finally:
         ctx.set_matvec_mode(MV_FP32_SIMT)
+
+
+@pytest.mark.parametrize("mode", [MV_SUBSET_EXACT, MV_BF16X3_TC])
+@pytest.mark.parametrize("scale", [1e-34, 1e-30, 1e30])
+def test_columns_of_extreme_magnitude(gpu_ctx, mode, scale):
+    """A column's digits scale with it over FP32's range, so K (s b) = s K b as far as FP32 holds both."""
+    n, m = 400, 700
+    bed, _ = synth.synth_bed(67, n, m, 0.02)
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    b = np.random.default_rng(5).standard_normal(n).astype(np.float32)
+    if mode == MV_BF16X3_TC:
+        ctx.grm_build(GRM_BF16X3_TC)
+    ctx.set_matvec_mode(mode)
+    try:
+        y = ctx.getCrossprodMatAndKin(b).astype(np.float64)
+        z = ctx.getCrossprodMatAndKin((b * np.float64(scale)).astype(np.float32)) / np.float64(scale)
+    finally:
+        ctx.set_matvec_mode(MV_FP32_SIMT)
+    assert np.abs(z - y).max() < 2 * TOL * np.abs(y).max()
