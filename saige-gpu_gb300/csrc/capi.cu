@@ -289,6 +289,7 @@ struct sg_ctx {
   double* d_gk_p2d = nullptr;
   float *d_gk_dp = nullptr, *d_gk_p2 = nullptr;
   bool gk_refused = false;
+  double digit_spread = 0.0;  // of the GRM markers' 1/sd^2 (see fp32_form)
   bool k_exact = false;     // K holds the FP32-class GRM (not the single-product BF16 one)
   // synthetic bed image
   uint8_t* d_synth = nullptr;
@@ -796,6 +797,14 @@ static int setgeno_core(sg_ctx* c, const uint8_t* raw, int64_t raw_pitch, int64_
       c->vr_index.push_back((int32_t)i);
     }
   }
+  double wmax = 0.0, inv_sum = 0.0;
+  for (const float x : c->invstd)
+    if (x > 0.0f) {
+      const double w = (double)x * (double)x;
+      wmax = std::max(wmax, w);
+      inv_sum += 1.0 / w;
+    }
+  c->digit_spread = wmax * inv_sum / (double)std::max<size_t>(c->invstd.size(), 1);
   c->fill_all.resize(m_bim);
   for (int64_t i = 0; i < m_bim; ++i) c->fill_all[i] = qc[i].fill;
   c->qc_min_maf = min_maf;
@@ -1532,12 +1541,23 @@ struct Fp32Scope {
 // G at 1.0 with five short kernels beside (n = 20,000, M = 30,000, one column: 0.46 against 0.13 ms).
 // Gemv: FP32 K streamed once per eight columns, in the FP32 engine (measured against its GEMM at the gemv
 // kernel); beyond 16 columns only while K stays near L2's size.
+//
+// A column is fixed-point at 2^-25 of its largest entry, so entries far below that keep fewer bits than BF16 halves
+// (2^-17 of each entry) would.  The operand at risk is T' = d' (G' v), which grows as sqrt(d') and is weighted by 1/sqrt(d')
+// in the result: its quantisation against the halves' is 0.045 sqrt(spread), spread = max d' mean(1/d') over the GRM
+// markers.  RMS error of K v in FP64 restatements of both (N = 20,000, M = 3,000; digits against halves): 0.06 at a spread of
+// 18 (MAF above 0.01), 0.19 at 157 (0.0005), 0.65 at 1,779 (0.0001), but 1.29 at 6,789 (1% of the markers carried three
+// times among common ones).  Beyond 512 the products stay with the engine's halves.  v itself needs no rule: the mean of
+// its quantisation leaves with the centring, and only a single entry above sqrt(N) times the rest costs more than the
+// halves do (1.1 times their error at N = 20,000; a unit vector 0.13).
+constexpr double kDigitSpread = 512.0;
 enum class Fp32Form { kEngine, kGenotypes, kGemv };
 static Fp32Form fp32_form(sg_ctx* c) {
   const Engine& e = c->eng;
   if (!e.fp32_cols || c->loco) return Fp32Form::kEngine;
-  if (c->mv_mode == SG_MV_SUBSET_EXACT) return fp4_ready(c) ? Fp32Form::kGenotypes : Fp32Form::kEngine;
-  if (c->mv_mode == SG_MV_BF16X3_TC && c->k_exact && !c->k_split && (double)c->m_qc <= 2.4 * (double)c->nn)
+  const bool digits = c->digit_spread <= kDigitSpread;
+  if (c->mv_mode == SG_MV_SUBSET_EXACT) return digits && fp4_ready(c) ? Fp32Form::kGenotypes : Fp32Form::kEngine;
+  if (c->mv_mode == SG_MV_BF16X3_TC && digits && c->k_exact && !c->k_split && (double)c->m_qc <= 2.4 * (double)c->nn)
     return fp4_cohort_ready(c) ? Fp32Form::kGenotypes : Fp32Form::kEngine;
   if (c->mv_mode == SG_MV_FP32_SIMT && !c->k_split && (e.fp32_cols <= 16 || e.np <= 8192)) return Fp32Form::kGemv;
   return Fp32Form::kEngine;

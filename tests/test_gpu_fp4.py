@@ -242,3 +242,27 @@ def test_columns_of_extreme_magnitude(gpu_ctx, mode, scale):
     finally:
         ctx.set_matvec_mode(MV_FP32_SIMT)
     assert np.abs(z - y).max() < 2 * TOL * np.abs(y).max()
+
+
+@pytest.mark.parametrize("singles", [0, 20])
+def test_rare_markers_keep_the_engine_products(gpu_ctx, singles):
+    """1/sd^2 of markers carried once among 6,000 samples is 3,000 times the others': the drop-ins' products stay with
+    the engine's BF16 halves, which keep each entry's own bits."""
+    n, m = 6000, 400
+    bed, _ = synth.synth_bed(78, n, m, 0.0)
+    raw = np.frombuffer(bed, np.uint8).copy()
+    rows = raw[3:].reshape(m, n // 4)
+    for k in range(singles):
+        rows[k] = 0xFF
+        rows[k, 7 * k] = 0xFE  # one copy
+    b = np.random.default_rng(6).standard_normal(n).astype(np.float32)
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(raw, n, m, min_maf=0.0)
+    ctx.set_matvec_mode(MV_SUBSET_EXACT)
+    try:
+        y, z = ctx.getCrossprodMatAndKin(b), ctx.grm_matmul(b).astype(np.float32)
+    finally:
+        ctx.set_matvec_mode(MV_FP32_SIMT)
+    assert np.array_equal(y, z) == (singles > 0)
+    assert np.abs(y - z).max() < 6e-5 * np.abs(z).max()
