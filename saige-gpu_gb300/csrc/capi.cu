@@ -1535,12 +1535,19 @@ struct Fp32Scope {
   bool outer = false;
 };
 
-// Forms of a drop-in's product.  Genotypes: exact integers through G on the FP4 pipe (k_fp4.cu) in the
-// subset-exact engine, and in the split-BF16 engine over an FP32-class K where G's two half-byte matrices (n
-// M bytes) are at most 0.6 of K's 4 n^2: K is then read at ~0.55 of the copy rate by the 32-column split GEMM,
-// G at 1.0 with five short kernels beside (n = 20,000, M = 30,000, one column: 0.46 against 0.13 ms).
-// Gemv: FP32 K streamed once per eight columns, in the FP32 engine (measured against its GEMM at the gemv
-// kernel); beyond 16 columns only while K stays near L2's size.
+// Forms of a drop-in's product, by the most columns a step of the call has.
+//
+// Genotypes: exact integers through G on the FP4 pipe (k_fp4.cu) in the subset-exact engine, and in the split-BF16 engine
+// over an FP32-class K: up to 64 columns, or at N < 1,024, where M <= 2.4 N (G's two half-byte matrices are then at most 0.6
+// of K's 4 N^2 bytes), beyond where M <= 0.6 N and N >= 6,000.  Products (ms, K's 16-bit halves against G): N = 24,576, M = 58,900 one
+// column 0.49 / 0.26, 64 0.52 / 0.46, but 128 0.57 / 0.69; N = 18,000, M = 10,800 one 0.21 / 0.09, 128 0.23 / 0.20, 256
+// 0.33 / 0.31.  K fits L2 below N ~ 6,000, and G's six kernels then take longer than its GEMM (N = 2,000, M = 4,800: 0.04 /
+// 0.07 at 64).  Up to 64 columns G is kept there too, for its 30 times smaller error: whole calls wait for the host more than
+// for either (128 columns of getSigma_X at 2,000 x 4,800 3.03 / 3.31 ms; at 500 x 1,200 2.17 / 2.43).
+//
+// Gemv: FP32 K streamed once per eight columns, in the FP32 engine: up to 16 columns, and while columns times N stays within
+// 2^19, 192 columns and N = 8,192.  Against the GEMM (ms): 61 columns at N = 8,192 0.56 / 0.96, 128 at 4,096 0.33 / 0.41,
+// 192 at 2,048 0.16 / 0.19; outside it 128 at 8,192 1.11 / 0.92, 256 at 4,096 0.67 / 0.58, 512 at 2,048 0.41 / 0.26.
 //
 // A column is fixed-point at 2^-25 of its largest entry, so entries far below that keep fewer bits than BF16 halves
 // (2^-17 of each entry) would.  The operand at risk is T' = d' (G' v), which grows as sqrt(d') and is weighted by 1/sqrt(d')
@@ -1551,15 +1558,24 @@ struct Fp32Scope {
 // its quantisation leaves with the centring, and only a single entry above sqrt(N) times the rest costs more than the
 // halves do (1.1 times their error at N = 20,000; a unit vector 0.13).
 constexpr double kDigitSpread = 512.0;
+namespace sg {
+bool fp32_through_genotypes(int64_t n, int64_t m, int64_t cols) {
+  return cols <= 64 || n < 1024 ? (double)m <= 2.4 * (double)n : n >= 6000 && (double)m <= 0.6 * (double)n;
+}
+bool fp32_by_gemv(int64_t np, int64_t cols) {
+  return cols <= 16 || (cols <= 192 && np <= 8192 && cols * np <= (1 << 19));
+}
+}  // namespace sg
+
 enum class Fp32Form { kEngine, kGenotypes, kGemv };
 static Fp32Form fp32_form(sg_ctx* c) {
   const Engine& e = c->eng;
   if (!e.fp32_cols || c->loco) return Fp32Form::kEngine;
   const bool digits = c->digit_spread <= kDigitSpread;
   if (c->mv_mode == SG_MV_SUBSET_EXACT) return digits && fp4_ready(c) ? Fp32Form::kGenotypes : Fp32Form::kEngine;
-  if (c->mv_mode == SG_MV_BF16X3_TC && digits && c->k_exact && !c->k_split && (double)c->m_qc <= 2.4 * (double)c->nn)
+  if (c->mv_mode == SG_MV_BF16X3_TC && digits && c->k_exact && !c->k_split && fp32_through_genotypes(c->nn, c->m_qc, e.fp32_cols))
     return fp4_cohort_ready(c) ? Fp32Form::kGenotypes : Fp32Form::kEngine;
-  if (c->mv_mode == SG_MV_FP32_SIMT && !c->k_split && (e.fp32_cols <= 16 || e.np <= 8192)) return Fp32Form::kGemv;
+  if (c->mv_mode == SG_MV_FP32_SIMT && !c->k_split && fp32_by_gemv(e.np, e.fp32_cols)) return Fp32Form::kGemv;
   return Fp32Form::kEngine;
 }
 

@@ -1,0 +1,32 @@
+"""Rules that choose a product's form by its sizes, as plain functions of the library (no GPU needed)."""
+import ctypes as C
+
+import pytest
+
+
+def rule(name, *args):
+    from saigegpu import build
+    fn = getattr(C.CDLL(build.build_lib()), name)
+    fn.restype = C.c_bool
+    return fn(*args)
+
+
+def i64(*v):
+    return [C.c_int64(x) for x in v]
+
+
+@pytest.mark.parametrize("n,m,cols,want", [
+    (20000, 30000, 1, True), (20000, 48000, 64, True), (20000, 48001, 64, False), (1000, 2400, 63, True), (1023, 2000, 256, True), (1024, 2000, 65, False),
+    (20000, 30000, 65, False), (20000, 12000, 65, True), (20000, 12000, 512, True), (20000, 12001, 65, False),
+    (6000, 3600, 128, True), (5999, 3000, 128, False)])
+def test_drop_ins_on_split_bf16_through_genotypes(n, m, cols, want):
+    """Wide calls leave the genotypes where K's GEMM is the faster one."""
+    assert rule("_ZN2sg22fp32_through_genotypesElll", *i64(n, m, cols)) is want
+
+
+@pytest.mark.parametrize("np_,cols,want", [
+    (128, 1, True), (24576, 16, True), (24576, 17, False), (8192, 64, True), (8192, 65, False), (8320, 17, False),
+    (4096, 128, True), (4096, 129, False), (2048, 192, True), (2048, 193, False), (1024, 512, False)])
+def test_drop_ins_on_fp32_by_gemv(np_, cols, want):
+    """Wide calls leave the few-column kernel where the GEMM is the faster one."""
+    assert rule("_ZN2sg12fp32_by_gemvEll", *i64(np_, cols)) is want
