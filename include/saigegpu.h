@@ -104,8 +104,10 @@ enum sg_tc_option {
   SG_TC_SYRK_GROUP = 3,  /* row tiles per raster group of the SYRK (1..4096); default 8 */
   SG_TC_GRMV_SLICE = 4,  /* K slice bytes per pipeline stage of the split-BF16 GRM.V: 0 = by
                             width (128 up to 160 columns, else 64), 64 or 128; default 0 */
-  SG_TC_SUBSET_PAIR = 5, /* the subset-exact engine's genotype GEMMs on CTA pairs: 0 never,
-                            1 always, 2 above 160 columns (default) */
+  SG_TC_SUBSET_PAIR = 5, /* the subset-exact engine's genotype GEMMs on CTA pairs: 0 never (tiles of
+                            up to 96 columns of SG_MV_SUBSET_EXACT then take two-bit genotypes, if there
+                            is memory for that copy), 1 always, 2 except where up to 96 columns take
+                            the two-bit genotypes (default) */
   SG_TC_SUBSET_SLICE = 6 /* their K slice bytes per pipeline stage: 0 = by width (128 up to 160
                             columns, else 64), 64, 128, 256 (default: two 128-byte boxes per
                             operand and stage) or 512 (four); a width without room for two such

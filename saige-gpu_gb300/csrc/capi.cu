@@ -2523,14 +2523,17 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
       return SG_OK;
     }
     const int64_t np = e.np, mg = c->mg;
-    const int64_t npad = tc_grmv_padded_cols(round_up(nact, 32), e.cap_cols, np, kTilesSplitB, c->num_sms);
-    SG_TRY(upload_list(c, npad));
     const size_t cap = (size_t)e.cap_cols;
     if (!e.Vb) SG_TRY(dev_alloc(c, &e.Vb, cap * np * 4));
     if (!e.Tm) SG_TRY(dev_alloc_t(c, &e.Tm, cap * mg));
     if (!e.Tb) SG_TRY(dev_alloc(c, &e.Tb, cap * mg * 4));
     if (!e.Um) SG_TRY(dev_alloc_t(c, &e.Um, cap * np));
     if (!e.spart) SG_TRY(dev_alloc_t(c, &e.spart, cap * (size_t)std::max(subset_nblk(np), subset_nblk(mg))));
+    const int64_t n32 = round_up(nact, 32);
+    const bool two_bit = c->mv_mode == SG_MV_SUBSET_EXACT && (tc_splitb_packed(np, n32) || tc_splitb_packed(mg, n32)) &&
+                         gpack_ready(c);
+    const int64_t npad = tc_grmv_padded_cols(n32, e.cap_cols, np, kTilesSplitB, c->num_sms, two_bit);
+    SG_TRY(upload_list(c, npad));
     uint16_t* vh = static_cast<uint16_t*>(e.Vb);
     uint16_t* vl = vh + cap * np;
     uint16_t* th = static_cast<uint16_t*>(e.Tb);
@@ -2565,9 +2568,8 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
     }
     launch_subset_prepare(e.Pf, np, e.d_gcols, npad, e.d_st, e.d_slots, e.winv, e.spart, vh, vl, c->stream);
     c->launches += 2;
-    const bool narrow = (tc_splitb_packed(np, npad) || tc_splitb_packed(mg, npad)) && gpack_ready(c);
-    const uint8_t* Pmm = narrow ? static_cast<const uint8_t*>(c->d_Gp) : nullptr;
-    const uint8_t* Psm = narrow ? Pmm + gpack_bytes(mg, np) : nullptr;
+    const uint8_t* Pmm = two_bit ? static_cast<const uint8_t*>(c->d_Gp) : nullptr;
+    const uint8_t* Psm = two_bit ? Pmm + gpack_bytes(mg, np) : nullptr;
     cudaError_t err = tc_gemm_splitb(Gmm, Pmm, mg, np, vh, vl, npad, e.Tm, mg, c->stream, false, 0);
     if (err != cudaSuccess) return set_err(c, SG_ERR_CUDA, "tcgen05 genotype GEMM (G'V): %s", cudaGetErrorString(err));
     launch_subset_scale(vh, vl, np, c->nn, e.d_gcols, npad, e.d_st, e.d_slots, e.max_w, e.Tm, mg, th, tl, e.spart,

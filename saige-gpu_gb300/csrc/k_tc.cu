@@ -960,7 +960,7 @@ static int g_opt[kTcOptions] = {
     512,  // kTcDrainBytes: bytes of K per row one TMEM accumulator takes before it is drained
     8,    // kTcSyrkGroup: row tiles per raster group of the SYRK
     0,    // kTcGrmvSlice: K slice bytes of the split-BF16 GRM.V (0: by width, 64 or 128)
-    2,    // kTcSubsetPair: subset-exact genotype GEMMs on CTA pairs (2: above 160 columns)
+    2,    // kTcSubsetPair: subset-exact genotype GEMMs on CTA pairs (2: where the two-bit form does not serve)
     256,  // kTcSubsetSlice: their K-stage bytes (0: 128 up to 160 columns, else 64; or 64 / 128 / 256 / 512)
 };
 
@@ -1148,16 +1148,18 @@ int tc_gemm_tile_n(int64_t ncols, int set) {
 // Few columns stay off CTA pairs and take their genotypes in two bits (tc_packed_kernel).  Measured per product
 // (two GEMMs) at N = 50,000, M = 100,000, two-bit form against CTA pairs on the BF16 one: 32 columns 1.38
 // against 3.00 ms, 64 1.98 against 3.15, 96 2.72 against 3.23, but 128 4.12 against 3.57 (and there at
-// N = 20,000, M = 30,000 0.74 against 0.64).  Single CTAs on the BF16 form were the slowest at each width.
+// N = 20,000, M = 30,000 0.74 against 0.64).
 constexpr int kPackMaxCols = 96;
 
-// CTA pairs for a subset-exact genotype GEMM over ncols columns: every width without the two-bit form (at
-// 160 columns 3.82 against 5.10 ms; at N = 100k, M = 150k, 256-byte K stages, pairs took 512 columns from
-// 49.7 to 32.8 ms and 1024 from 89.4 to 61.8 ms).
-static bool subset_pair(int64_t ncols) {
+// CTA pairs for a subset-exact genotype GEMM over ncols columns: every width but those that the two-bit form takes, if
+// it is there (two_bit: BF16 halves, and memory for the copy).  Single CTAs against pairs at N = 50,000, M = 100,000: BF16
+// 3.38 / 3.08 ms at 32 columns, 3.63 / 3.22 at 64, 4.19 / 3.30 at 96, 5.10 / 3.82 at 160; FP16 / E4M3 4.56 / 4.43 at 32, 5.10
+// / 4.70 at 96, 5.24 / 4.78 at 128, and within 0.4% of each other at 64, 160 and 192.  At N = 100k, M = 150k, 256-byte K stages,
+// pairs took 512 BF16 columns from 49.7 to 32.8 ms and 1024 from 89.4 to 61.8 ms.
+bool tc_subset_pair(int64_t ncols, bool two_bit) {
   for (const GrmvChoice& b : g_subset_plan)
     if (ncols <= b.max_cols) return b.pair != 0;
-  return g_opt[kTcSubsetPair] == 2 ? ncols > kPackMaxCols : g_opt[kTcSubsetPair] != 0;
+  return g_opt[kTcSubsetPair] == 2 ? !two_bit || ncols > kPackMaxCols : g_opt[kTcSubsetPair] != 0;
 }
 
 static int subset_slice(int64_t ncols) {
@@ -1180,21 +1182,21 @@ static int splitb_stage_bytes(int RB, int BN, bool pair) {
 // bounds these kernels, over the fraction of the last wave of 1-tile-per-SM(-pair) tiles that is
 // busy): padded * (A bytes per stage / BN + B bytes per stage per column) / wave_efficiency; a CTA
 // pair loads half of the B tile per SM and fills num_sms / 2 tile slots per wave.
-int64_t tc_grmv_padded_cols(int64_t ncols32, int64_t cap, int64_t np, int set, int num_sms) {
+int64_t tc_grmv_padded_cols(int64_t ncols32, int64_t cap, int64_t np, int set, int num_sms, bool two_bit) {
   double best = 1e300;
   int64_t best_cols = ncols32;
   for (int w : tile_widths(set)) {
     const int64_t padded = (ncols32 + w - 1) / w * w;
     if (padded > cap) continue;
     const bool pair = (set == kTilesSplitBF16 && grmv_choice(padded).pair != 0) ||
-                      (set == kTilesSplitB && subset_pair(padded));
+                      (set == kTilesSplitB && tc_subset_pair(padded, two_bit));
     const int64_t nrt = pair ? (np / kTileM + 1) / 2 : np / kTileM;
     const int64_t slots = pair ? num_sms / 2 : num_sms;
     const int bn = tc_gemm_tile_n(padded, set);
     const int64_t tiles = nrt * (padded / bn);
     const int64_t waves = (tiles + slots - 1) / slots;
     const double eff = (double)tiles / (double)(waves * slots);
-    const bool packed = set == kTilesSplitB && !pair && bn <= kPackMaxCols;  // an eighth of the A bytes
+    const bool packed = two_bit && !pair && bn <= kPackMaxCols;  // an eighth of the A bytes
     const double cost = (double)padded * ((double)kATileBytes / (packed ? 8 : 1) / bn + (double)kRowBytes / (pair ? 2 : 1)) / eff;
     if (cost < best) {
       best = cost;
@@ -1409,7 +1411,7 @@ cudaError_t tc_gemm_bf16x3(const void* Kh, const void* Kl, int64_t np, const voi
 }
 
 bool tc_splitb_packed(int64_t kdim, int64_t ncols) {
-  return !subset_pair(ncols) && tc_gemm_tile_n(ncols, kTilesSplitB) <= kPackMaxCols && kdim % kPackK == 0 &&
+  return !tc_subset_pair(ncols, true) && tc_gemm_tile_n(ncols, kTilesSplitB) <= kPackMaxCols && kdim % kPackK == 0 &&
          g_opt[kTcDrainBytes] % (2 * kPackK) == 0;
 }
 
@@ -1438,7 +1440,7 @@ cudaError_t tc_gemm_splitb(const void* A, const void* A2bit, int64_t rows, int64
     if (e != cudaSuccess) return e;
     return check ? check_error_flag(s) : cudaSuccess;
   }
-  const bool pair = subset_pair(ncols);
+  const bool pair = tc_subset_pair(ncols, A2bit != nullptr);
   int RB = splitb_stage_bytes(subset_slice(ncols), BN, pair);
   while (RB > 128 && kdim % (RB / 2) != 0) RB /= 2;  // whole stages over K
   const int box = RB > 128 ? 128 : RB;  // a 256- or 512-byte stage is 2 or 4 128-byte boxes per operand
@@ -1569,7 +1571,7 @@ cudaError_t tc_gemm_splitb8(const void* A, const void* A8, int64_t rows, int64_t
       site < 0 || site > 1)
     return cudaErrorInvalidValue;
   const int BN = tc_gemm_tile_n(ncols, kTilesSplitB);
-  const bool pair = subset_pair(ncols) || BN > 160;
+  const bool pair = tc_subset_pair(ncols, false) || BN > 160;
   const int brows = pair ? BN / 2 : BN;
   CUtensorMap a, b, a8, b8;
   if (!make_map_dt(&a, A, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, kdim, rows, (uint64_t)kdim * 2, kTileM, 128) ||

@@ -142,7 +142,10 @@ enum { kTilesPlain = 0, kTilesSplitTF32 = 1, kTilesSplitBF16 = 2, kTilesSplitB =
 // site (0 or 1): which of two call sites queued back to back on one stream (own tile tables).
 cudaError_t tc_gemm_splitb(const void* A, const void* A2bit, int64_t rows, int64_t kdim, const void* Bh, const void* Bl,
                            int64_t ncols, float* D, int64_t ldd, cudaStream_t s, bool check, int site);
+// whether a GEMM with the two-bit copy at hand takes it
 bool tc_splitb_packed(int64_t kdim, int64_t ncols);
+// whether a subset-exact GEMM runs on CTA pairs, with (two_bit) or without that copy
+bool tc_subset_pair(int64_t ncols, bool two_bit);
 // The same with FP16 high halves and E4M3 low halves (A in FP16 and in E4M3, kdim a multiple of 128)
 cudaError_t tc_gemm_splitb8(const void* A, const void* A8, int64_t rows, int64_t kdim, const void* Bh,
                             const void* Bl8, int64_t ncols, float* D, int64_t ldd, cudaStream_t s, bool check,
@@ -151,7 +154,7 @@ cudaError_t tc_gemm_splitb8(const void* A, const void* A8, int64_t rows, int64_t
 int tc_gemm_tile_n(int64_t ncols, int set);
 // Columns a GRM.V launch covers for ncols live columns (a multiple of 32, or of 16 for split-BF16),
 // padded to the width a cost model picks, at most cap.
-int64_t tc_grmv_padded_cols(int64_t ncols, int64_t cap, int64_t np, int set, int num_sms);
+int64_t tc_grmv_padded_cols(int64_t ncols, int64_t cap, int64_t np, int set, int num_sms, bool two_bit = false);
 // Split-TF32 GRM.V that allocates nothing: scratch in a static device array (k_tc.cu).
 int64_t tc_noalloc_max_elems();
 cudaError_t tc_gemm_tf32x3_noalloc(const float* Khi, const float* Klo, int64_t np, const float* P,

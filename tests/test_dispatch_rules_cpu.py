@@ -30,3 +30,10 @@ def test_drop_ins_on_split_bf16_through_genotypes(n, m, cols, want):
 def test_drop_ins_on_fp32_by_gemv(np_, cols, want):
     """Wide calls leave the few-column kernel where the GEMM is the faster one."""
     assert rule("_ZN2sg12fp32_by_gemvEll", *i64(np_, cols)) is want
+
+
+@pytest.mark.parametrize("cols,two_bit,want", [(32, True, False), (96, True, False), (128, True, True), (32, False, True),
+                                               (96, False, True), (160, False, True), (512, True, True)])
+def test_pairs_wherever_the_two_bit_form_does_not_serve(cols, two_bit, want):
+    """Without the two-bit copy (refused memory, or the FP16 / E4M3 form) single CTAs are the slower ones."""
+    assert rule("_ZN2sg14tc_subset_pairElb", C.c_int64(cols), C.c_bool(two_bit)) is want
