@@ -919,6 +919,31 @@ static int bed_upload(sg_ctx* c, const uint8_t* body, int64_t nb, int64_t m, int
   return SG_OK;
 }
 
+namespace sg {
+// Whether a kernel on ``device`` may read memory that cudaPointerGetAttributes describes so: its own device's, or managed.
+// Another device's (without peer access) and what else a copy can read go through a copy.
+bool kernel_reads(int type, int where, int device) {
+  return type == cudaMemoryTypeManaged || (type == cudaMemoryTypeDevice && where == device);
+}
+}  // namespace sg
+
+// The same from device memory, re-pitched in place where this device's kernels can read it.
+static int bed_copy(sg_ctx* c, const uint8_t* body, int64_t nb, int64_t m, int64_t n_fam, uint8_t* raw,
+                    int64_t raw_pitch) {
+  if (m == 0) return SG_OK;
+  cudaPointerAttributes at{};
+  const bool known = cudaPointerGetAttributes(&at, body) == cudaSuccess;
+  cudaGetLastError();
+  if (known && kernel_reads(at.type, at.device, c->device)) {
+    launch_bed_pitch(body, body + nb * m, nb, m, n_fam, raw, raw_pitch, c->stream);
+    SG_LAUNCHED(c, 1);
+    return SG_OK;
+  }
+  SG_CUDA(c, cudaMemsetAsync(raw, 0, raw_pitch * m, c->stream));
+  SG_CUDA(c, cudaMemcpy2DAsync(raw, raw_pitch, body, nb, nb, m, cudaMemcpyDeviceToDevice, c->stream));
+  return SG_OK;
+}
+
 static int setgeno_common(sg_ctx* c, const uint8_t* bed, bool on_device, uint64_t bed_len,
                           int64_t n_fam, int64_t m_bim, const int32_t* sub_1based, int64_t n_sub,
                           const uint8_t* pheno_mask, float min_maf, float max_missing,
@@ -944,15 +969,11 @@ static int setgeno_common(sg_ctx* c, const uint8_t* bed, bool on_device, uint64_
   const int64_t raw_pitch = round_up(std::max<int64_t>(nb, 1), kPitchAlign);
   uint8_t* raw = nullptr;
   SG_TRY(dev_alloc_t(c, &raw, (size_t)std::max<int64_t>(raw_pitch * m_bim, 16)));
-  if (on_device) {
-    launch_bed_pitch(bed + 3, bed + 3 + nb * m_bim, nb, m_bim, n_fam, raw, raw_pitch, c->stream);
-    SG_LAUNCHED(c, m_bim ? 1 : 0);
-  } else {
-    const int rc_up = bed_upload(c, bed + 3, nb, m_bim, n_fam, raw, raw_pitch);
-    if (rc_up != SG_OK) {
-      dev_free(c, raw);
-      return rc_up;
-    }
+  const int rc_up = on_device ? bed_copy(c, bed + 3, nb, m_bim, n_fam, raw, raw_pitch)
+                              : bed_upload(c, bed + 3, nb, m_bim, n_fam, raw, raw_pitch);
+  if (rc_up != SG_OK) {
+    dev_free(c, raw);
+    return rc_up;
   }
   int rc = setgeno_core(c, raw, raw_pitch, n_fam, m_bim, sub_1based, n_sub, pheno_mask, min_maf,
                         max_missing, vr_markers, n_vr, min_mac_vr, is_var_ratio, is_diag_one);

@@ -37,3 +37,10 @@ def test_drop_ins_on_fp32_by_gemv(np_, cols, want):
 def test_pairs_wherever_the_two_bit_form_does_not_serve(cols, two_bit, want):
     """Without the two-bit copy (refused memory, or the FP16 / E4M3 form) single CTAs are the slower ones."""
     assert rule("_ZN2sg14tc_subset_pairElb", C.c_int64(cols), C.c_bool(two_bit)) is want
+
+
+@pytest.mark.parametrize("kind,where,want", [(2, 1, True), (2, 0, False), (3, 0, True), (1, 1, False), (0, -2, False)])
+def test_which_images_a_kernel_reads(kind, where, want):
+    """A .bed image in this device's memory or in managed memory is re-pitched in place; one on another device, or in host
+    memory, goes through a copy.  kind: cudaMemoryType (0 unregistered, 1 host, 2 device, 3 managed)."""
+    assert rule("_ZN2sg12kernel_readsEiii", C.c_int(kind), C.c_int(where), C.c_int(1)) is want

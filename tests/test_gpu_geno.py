@@ -89,3 +89,16 @@ def test_host_and_device_images_give_the_same_genotypes(gpu_ctx, n, m):
     if n * m < 10000:
         o = plink.setgeno(host.tobytes(), n, m, np.arange(1, n + 1), np.ones(n, bool), 0.0, 1.0)
         np.testing.assert_array_equal(packed, plink.pack_codes(o.codes))
+
+
+@pytest.mark.parametrize("n,m", [(33, 40), (1030, 700)])
+def test_images_a_kernel_does_not_read_in_place(gpu_ctx, n, m):
+    """setgeno_device() of an image in pinned host memory (which a device-to-device copy takes) equals setgeno()."""
+    torch = pytest.importorskip("torch")
+    bed, _ = synth.synth_bed(5, n, m, 0.03)
+    gpu_ctx.setgeno(bed, n, m)
+    want = gpu_ctx.allele_freq(), gpu_ctx.packed_geno(), gpu_ctx.grm_diag()
+    image = torch.from_numpy(np.frombuffer(bed, np.uint8).copy()).pin_memory()
+    gpu_ctx.setgeno_device(image.data_ptr(), image.numel(), n, m)
+    for a, b in zip(want, (gpu_ctx.allele_freq(), gpu_ctx.packed_geno(), gpu_ctx.grm_diag())):
+        np.testing.assert_array_equal(a, b)
