@@ -1198,12 +1198,17 @@ extern "C" int sg_grm_build(sg_ctx* c, int precision) {
   if (!c->d_K) SG_TRY(dev_alloc_t(c, &c->d_K, (size_t)(np * np)));
   const float scale = 1.0f / (float)c->m_qc;
   if (precision != SG_GRM_BF16_TC && tc_available()) {
-    // exact integers on the FP4 pipe (k_fp4.cu) while 1/sd^2 spans at most a factor of 200 (MAF above
-    // ~0.0013): the markers of the smallest 1/sd^2 then keep a relative error of 6e-6 at most, that is
-    // off-diagonal entries within 1.6e-8 at M = 150k, as the FP32 build's were (4.1e-8: split BF16)
+    // Exact integers on the FP4 pipe (k_fp4.cu) where their rounding of 1/sd^2, common to all markers, costs no more than
+    // the other build's own: while 1/sd^2 spans at most a factor of 200 (MAF above ~0.0013) and its ``spread``, max D times
+    // the RMS of 1/D, is bounded.  Off-diagonal entries are then off by 4.9e-8 spread / sqrt(M) RMS.  Split BF16: 16-bit
+    // genotypes are off by 4.3e-6 / sqrt(M), so a spread of 80.  FP32: a chain of M FP32 sums is off by 2e-8 whatever M, so
+    // 0.6 sqrt(M), and where that is below 24 (common markers, MAF above 0.01) 24 from 128 markers on: the chain's largest
+    // error, on the diagonal, is the larger one from there (M = 300: 8e-7 against 3e-7, off-diagonals 2e-8 against 5e-8 RMS;
+    // M = 700 with one marker of MAF 0.0013, spread 136: off-diagonals 2e-8 against 25e-8, left to FP32).
     std::vector<double> weight, centre;
     grm_weights(c, precision, weight, centre);
-    const Fp4SyrkPlan plan = fp4_syrk_plan(weight.data(), c->m_qc, np, 200.0);
+    const Fp4SyrkPlan plan =
+        fp4_syrk_plan(weight.data(), c->m_qc, np, 200.0, fp4_syrk_spread(c->m_qc, precision == SG_GRM_BF16X3_TC));
     void* scratch = nullptr;
     const std::string err = c->err;
     if (plan.ok && dev_alloc(c, &scratch, (size_t)plan.bytes) == SG_OK) {

@@ -266,3 +266,27 @@ def test_rare_markers_keep_the_engine_products(gpu_ctx, singles):
         ctx.set_matvec_mode(MV_FP32_SIMT)
     assert np.array_equal(y, z) == (singles > 0)
     assert np.abs(y - z).max() < 6e-5 * np.abs(z).max()
+
+
+@pytest.mark.parametrize("m,rare", [(40, 0), (300, 1)])
+def test_fp32_grm_of_few_markers_keeps_the_weights_precision(gpu_ctx, m, rare):
+    """Few markers, one of them near the frequency bound: 1/sd^2 as integers of one exponent would cost the common
+    markers' bits, so FP32 genotypes are multiplied.  Off-diagonal entries: 2^-24 on each of a term's two factors and of
+    the chain's sums, over M terms of order one (a root of M over M), with room for the oracle's FP32 genotypes."""
+    n = 2000
+    bed, _ = synth.synth_bed(88, n, m, 0.0)
+    raw = np.frombuffer(bed, np.uint8).copy()
+    rows = raw[3:].reshape(m, n // 4)
+    for k in range(rare):
+        rows[k] = 0xFF
+        rows[k, :6] = 0xFE  # one copy in six samples: MAF 0.0015
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(raw, n, m, min_maf=0.001)
+    g = plink.setgeno(raw.tobytes(), n, m, np.arange(1, n + 1), np.ones(n, bool), 0.001, 0.15)
+    ref = aireml.DenseGRM(g).K
+    ctx.grm_build(GRM_FP32_SIMT)
+    assert ctx.build_timing()["zbuild_ms"] > 0  # FP32 genotypes were written out
+    off = ~np.eye(n, dtype=bool)
+    err = (ctx.grm_get() - ref)[off]
+    assert np.sqrt((err ** 2).mean()) < 16 * 2.0 ** -24 / np.sqrt(m)
