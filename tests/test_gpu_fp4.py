@@ -290,3 +290,33 @@ def test_fp32_grm_of_few_markers_keeps_the_weights_precision(gpu_ctx, m, rare):
     off = ~np.eye(n, dtype=bool)
     err = (ctx.grm_get() - ref)[off]
     assert np.sqrt((err ** 2).mean()) < 16 * 2.0 ** -24 / np.sqrt(m)
+
+
+def test_products_over_changed_fills(gpu_ctx):
+    """setgeno with a sample list but every sample in the phenotype mask: its fills of missing calls are counted over all
+    of them, and the drop-ins' subset, the listed samples, has its own at some markers (the fill-change terms)."""
+    n_fam, m = 1000, 1500
+    bed, _ = synth.synth_bed(93, n_fam, m, 0.1)
+    sub = np.sort(np.random.default_rng(8).permutation(n_fam)[:517]).astype(np.int32) + 1
+    codes = plink.decode_bed(bed, n_fam, m)  # 3: missing
+    miss, allele = (codes == 3).sum(1), np.where(codes == 3, 0, codes).sum(1)
+    fill_all = np.floor(2 * (allele / (2.0 * (len(sub) - miss))) + 0.5)
+    c = codes[:, sub - 1]
+    miss, allele = (c == 3).sum(1), np.where(c == 3, 0, c).sum(1)
+    fill = np.floor(2 * (allele / (2.0 * (len(sub) - miss))) + 0.5)
+    assert ((fill_all != fill) & (miss > 0)).sum() > 100  # more than one word of the fill-change bit map
+    mask = np.zeros(n_fam, bool)
+    mask[sub - 1] = True
+    g = plink.setgeno(bed, n_fam, m, sub, mask, 0.01, 0.15)
+    b = np.random.default_rng(9).standard_normal(len(sub)).astype(np.float32)
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n_fam, m, sub)
+    ctx.set_matvec_mode(MV_SUBSET_EXACT)
+    try:
+        y, z = ctx.getCrossprodMatAndKin(b), ctx.grm_matmul(b)
+    finally:
+        ctx.set_matvec_mode(MV_FP32_SIMT)
+    want = aireml.DenseGRM(g).K @ b.astype(np.float64)
+    assert np.abs(y - want).max() < TOL * np.abs(want).max()
+    assert np.abs(z - want).max() < 8 * 2.0 ** -17 * np.abs(want).max()
