@@ -3,7 +3,7 @@ on CTA pairs: the same products in the same order, so the same bits."""
 import numpy as np
 import pytest
 
-from saigegpu import MV_FP32_SIMT, MV_SUBSET_EXACT, TC_SUBSET_PAIR, Context, SaigeGpuError, synth
+from saigegpu import MV_FP32_SIMT, MV_SUBSET_EXACT, TC_DRAIN_BYTES, TC_SUBSET_PAIR, Context, SaigeGpuError, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -168,3 +168,35 @@ def test_more_row_blocks_than_a_grid_has_rows(gpu_ctx):
         ctx.set_matvec_mode(MV_FP32_SIMT)
         bed, _ = synth.synth_bed(9, 64, 90, 0.02)
         ctx.setgeno(bed, 64, 90)  # the 4 GB of genotypes leave the shared context
+
+
+@pytest.mark.parametrize("drain", [256, 512, 2048])
+def test_same_bits_at_several_column_tiles(gpu_ctx, drain):
+    """Three column tiles of 96 (single CTAs asked for) and other drain lengths, past a whole number of drains."""
+    n, m, k = 900, 1500, 288
+    ctx = gpu_ctx
+    bed, _ = synth.synth_bed(51, n, m, 0.05)
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    V = np.random.default_rng(k).standard_normal((n, k)) * 10.0 ** np.linspace(-18, 18, k)
+    prev = ctx.tc_options()
+    try:
+        ctx.set_matvec_mode(MV_SUBSET_EXACT)
+        ctx.engine_reserve(320, 1)
+        ctx.set_tc_option(TC_DRAIN_BYTES, drain)
+        out = []
+        for pair in (1, 0):
+            ctx.set_tc_option(TC_SUBSET_PAIR, pair)
+            ctx.engine_set_pheno(0, np.ones(n), np.array([1.0, 0.5]))
+            ids = [int(i) for i in ctx.engine_submit(0, 1, V)]
+            ctx.engine_reset_timing()
+            ctx.engine_hold_results(True)
+            ctx.engine_run()
+            assert len(ctx.engine_step_trace()) == 1  # one launch over all of them
+            out.append(np.column_stack([ctx.engine_fetch(i)[0] for i in ids]))
+        np.testing.assert_array_equal(out[0], out[1])
+        assert np.isfinite(out[0]).all() and np.abs(out[0]).max(0).min() > 0
+    finally:
+        ctx.engine_hold_results(False)
+        ctx.set_tc_options(prev)
+        ctx.set_matvec_mode(MV_FP32_SIMT)
