@@ -403,7 +403,7 @@ cudaError_t launch_fp4(const CUtensorMap& a, const CUtensorMap& b, int stages, i
   auto k = fp4_gemm_kernel<CT, S, kMode>;
   constexpr size_t sm = (size_t)S * (kAStage + 336 * CT) + 128 + 256;
   static_assert(sm <= 232448 && 2 * S + 4 <= 31, "stage ring and barriers fit the CTA's shared memory");
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = set_dynamic_smem(reinterpret_cast<const void*>(k), sm);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * ntiles));
@@ -526,7 +526,7 @@ cudaError_t launch_fp4_gbuild(const uint8_t* codes, int64_t pitch, const int32_t
                               void* Gsm, cudaStream_t s) {
   const int64_t m1 = m > 0 ? m : 1;  // a cohort without markers still has its (zero) row blocks
   const int64_t rm = (m1 + 255) / 256 * 2, rs = (nn + 255) / 256 * 2;
-  const cudaError_t e = cudaFuncSetAttribute(fp4_gbuild_mm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMmSmem);
+  const cudaError_t e = tc::set_dynamic_smem(reinterpret_cast<const void*>(fp4_gbuild_mm_kernel), kMmSmem);
   if (e != cudaSuccess) return e;
   const int sn = fp4_stages(nn);
   dim3 g1((unsigned)((sn + kMmStages - 1) / kMmStages), (unsigned)(rm < 65535 ? rm : 65535),

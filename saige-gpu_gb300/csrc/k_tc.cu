@@ -716,7 +716,7 @@ cudaError_t launch_packed(const uint8_t* A, const CUtensorMap& b, const CUtensor
   auto k = tc_packed_kernel<BN, S, kBufs, kCtas, kExp>;
   constexpr size_t sm = (size_t)S * (kPackABytes + 4 * BN * kPackK) + 1024 + 256;
   static_assert((sm + 1024) * kCtas <= 233472 && 2 * S + kBufs + 6 <= 31, "kCtas CTAs' stages and barriers fit the SM");
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = set_dynamic_smem(reinterpret_cast<const void*>(k), sm);
   if (e != cudaSuccess) return e;
   k<<<(unsigned)(rows / kTileM * ncolt), 32 * (kExp + 6), sm, s>>>(A, b, b2, stages, drain, ncolt, D, ldd);
   return cudaGetLastError();
@@ -778,7 +778,7 @@ cudaError_t launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap
   static_assert(sm <= 232448, "stage ring exceeds the 227 KB of dynamic shared memory per CTA");
   static_assert(2 * S + 5 <= 31, "barriers, TMEM slot and abort flag fit the 256-byte tail");
   if (drain_kb < 1) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = set_dynamic_smem(reinterpret_cast<const void*>(k), sm);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ntiles * (kPair ? 2u : 1u));

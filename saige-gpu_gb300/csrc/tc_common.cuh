@@ -14,6 +14,13 @@ namespace tc {
 PFN_cuTensorMapEncodeTiled_v12000 tc_encode_fn();
 int* tc_error_flag();
 
+// Dynamic shared memory of a kernel about to be launched.  An earlier launch's error comes back first: setting the
+// attribute clears it unread (CUDA 13.0), and that launch's output would be taken for written.
+inline cudaError_t set_dynamic_smem(const void* kernel, size_t bytes) {
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 constexpr unsigned long long kWaitBudgetNs = 4000000000ull;  // 4 s per wait
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

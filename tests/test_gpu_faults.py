@@ -112,3 +112,24 @@ def test_a_step_whose_wait_ran_out_fails(cleared):
         for i in ids:
             ctx.engine_cancel(i)
         np.testing.assert_allclose(ctx.grm_matmul(V), ctx.grm_matmul(V), rtol=0, atol=0)  # still usable
+
+
+def test_a_launch_that_failed_is_reported_by_the_next_one():
+    """A launch with too many grid rows (refused by the runtime: nothing runs) before one that first sets its kernel's
+    shared memory, which would clear the error unread."""
+    torch = pytest.importorskip("torch")
+    with Context(0) as ctx:
+        ctx.make_current()
+        lib, buf = ctx._L, torch.zeros(4 << 16, dtype=torch.uint8, device="cuda:0")
+        torch.cuda.synchronize()
+        at = [C.c_void_p(buf.data_ptr() + (k << 16)) for k in range(4)]
+        gemv = lib._ZN2sg17launch_gemv_multiEPKflS1_PKilPfP11CUstream_st
+        gemv.restype = None
+        build = lib._ZN2sg17launch_fp4_gbuildEPKhlPKillPvS4_P11CUstream_st
+        # one marker of 16 samples: one stage of two row blocks each way, 24,576 bytes
+        args = (at[0], C.c_int64(16), at[1], C.c_int64(1), C.c_int64(16), at[2], at[3], C.c_void_p(0))
+        assert build(*args) == 0
+        gemv(at[0], C.c_int64(128), at[1], at[2], C.c_int64(8 * 65536), at[3], C.c_void_p(0))
+        assert build(*args) != 0
+        assert build(*args) == 0
+        torch.cuda.synchronize()
