@@ -2496,10 +2496,11 @@ static int engine_gemm_full(sg_ctx* c, int64_t ncols, bool* used_yf, int64_t* la
     if (form == Fp32Form::kGemv) {
       launch_gemv_multi(c->d_K, e.np, e.Pf, e.d_gcols, nact, e.Yf, c->stream);
     } else {
+      // drop-ins have slot 0 only: other slots' fill changes launch nothing
       const int64_t m = subset ? c->m_bim : c->m_qc, mg = subset ? c->mg : round_up(m, kRowTile);
       const uint8_t* g = static_cast<const uint8_t*>(subset ? c->d_G4 : c->d_Gk);
       const cudaError_t err = fp4_product(g, g + fp4_matrix_bytes(mg, c->nn), e.Pf, e.np, c->nn, mg, m, e.d_gcols, npad, ct,
-                                          e.d_st, subset ? e.d_slots : c->d_gk_slot, e.winv, subset ? e.max_w : 0, e.f4,
+                                          e.d_st, subset ? e.d_slots : c->d_gk_slot, e.winv, subset ? e.sub[0].dev.W : 0, e.f4,
                                           e.Yf, c->stream, &nl);
       if (err != cudaSuccess) return set_err(c, SG_ERR_CUDA, "tcgen05 genotype GEMM: %s", cudaGetErrorString(err));
       *launched = npad;

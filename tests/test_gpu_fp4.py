@@ -320,3 +320,29 @@ def test_products_over_changed_fills(gpu_ctx):
     want = aireml.DenseGRM(g).K @ b.astype(np.float64)
     assert np.abs(y - want).max() < TOL * np.abs(want).max()
     assert np.abs(z - want).max() < 8 * 2.0 ** -17 * np.abs(want).max()
+
+
+def test_other_slots_fill_changes_launch_nothing(gpu_ctx):
+    """A drop-in beside a slot that holds a masked subset with fill changes: as many kernels as without it."""
+    n, m = 600, 900
+    bed, _ = synth.synth_bed(95, n, m, 0.1)
+    ctx = gpu_ctx
+    ctx.set_matvec_mode(MV_FP32_SIMT)
+    ctx.setgeno(bed, n, m)
+    b = np.random.default_rng(2).standard_normal(n).astype(np.float32)
+    ctx.set_matvec_mode(MV_SUBSET_EXACT)
+    try:
+        ctx.engine_reserve(128, 2)
+        count, out = [], []
+        for masked in (False, True):
+            if masked:
+                ctx.engine_set_pheno(1, np.ones(n), np.array([0.6, 0.4]), np.arange(n) % 3 > 0)
+            for _ in range(2):
+                before = ctx.kernel_launches()
+                out.append(ctx.getCrossprodMatAndKin(b))
+                count.append(ctx.kernel_launches() - before)
+        assert count[1] == count[3]
+        for y in out:
+            np.testing.assert_array_equal(y, out[0])
+    finally:
+        ctx.set_matvec_mode(MV_FP32_SIMT)
