@@ -42,12 +42,17 @@ enum sg_status {
 
 /* GRM build precisions (sg_grm_build) */
 enum sg_grm_precision {
-  SG_GRM_FP32_SIMT = 0, /* near-exact FP32 K: exact integer sums on the FP4 tensor pipe, rounded once, while
-                           the GRM markers' 1/sd^2 span at most a factor of 200; else FP32 standardised
-                           genotypes, FP32 CUDA-core SYRK */
+  SG_GRM_FP32_SIMT = 0, /* FP32 K: exact integer sums on the FP4 tensor pipe, rounded to FP32 and scaled
+                           there, while 1/sd^2 in integers of one exponent costs the entries no more
+                           than FP32 genotypes do (the GRM markers' 1/sd^2 span at most a factor of 200,
+                           and less where they are few); else FP32 standardised genotypes, FP32
+                           CUDA-core SYRK */
   SG_GRM_BF16_TC = 1,   /* BF16 genotypes, tcgen05 SYRK, FP32 accumulation in TMEM */
-  SG_GRM_BF16X3_TC = 2  /* as SG_GRM_FP32_SIMT, with a split-BF16 (hi+lo, 4 products) tcgen05 SYRK over
-                           16-bit genotypes in the place of the CUDA-core one */
+  SG_GRM_BF16X3_TC = 2  /* K of 16-bit standardised genotypes (BF16 hi + lo): exact integer sums likewise,
+                           on the line through each marker's three rounded values (4e-8 RMS from their
+                           four products); else those products in a tcgen05 SYRK.  Off-diagonal entries
+                           are 4e-6 of their RMS from the unrounded genotypes', which the FP32 drop-ins
+                           in SG_MV_BF16X3_TC multiply where they go through the genotypes */
 };
 
 /* GRM.V product engines used inside the PCG (sg_set_matvec_mode) */
@@ -66,7 +71,9 @@ enum sg_matvec_mode {
                             436-495), applied through the genotype matrix (0/1/2 in BF16, exact)
                             with two tcgen05 GEMMs of two BF16 products each; needs no sg_grm_build.
                             The FP32 drop-ins run the same two products exactly, on integer digits
-                            of the vectors (kind::mxf4, G in E2M1 beside the BF16 one).
+                            of the vectors (kind::mxf4, G in E2M1 beside the BF16 one), unless rare
+                            markers without a frequency bound spread 1/sd^2 too far for one exponent
+                            a column.
                             The other engines restrict the cohort GRM to the subset instead */,
   SG_MV_SUBSET_EXACT_F8 = 6 /* the subset-exact engine with FP16 high halves (kind::f16) and E4M3
                             low halves (kind::f8f6f4, twice the FP16 rate) of each column scaled
@@ -78,6 +85,10 @@ enum sg_matvec_mode {
 };
 
 /* ------------------------------------------------------------ context */
+/* hbm_budget_bytes: the most this context allocates (0: no limit).  Beside G the engines build
+ * copies of it that only save time, at the first product that reads one: E2M1 (1 byte a sample and
+ * marker, both layouts) and two bits (1/2).  They give way to this context's other allocations, not
+ * to another library's in the process: a budget leaves room for those. */
 int sg_ctx_create(int device, uint64_t hbm_budget_bytes, sg_ctx **out);
 void sg_ctx_destroy(sg_ctx *ctx);
 /* Make the context's GPU current on the calling host thread; a caller that drives one context
@@ -158,7 +169,8 @@ int sg_setgeno_files(sg_ctx *ctx, const char *bed_path, const char *bim_path, co
                      const int32_t *sub_1based, int64_t n_sub, const uint8_t *pheno_mask,
                      float min_maf, float max_missing, const int32_t *vr_random_markers,
                      int64_t n_vr_random, float min_mac_vr, int is_var_ratio, int is_diag_one);
-/* Uses a .bed image already in device memory (e.g. from sg_synth_bed). */
+/* Uses a .bed image already in device memory (e.g. from sg_synth_bed): this device's or managed memory is
+ * read in place, any other that a device-to-device copy takes goes through one. */
 int sg_setgeno_device(sg_ctx *ctx, const uint8_t *bed_dev, uint64_t bed_len, int64_t n_fam,
                       int64_t m_bim, const int32_t *sub_1based, int64_t n_sub,
                       const uint8_t *pheno_mask, float min_maf, float max_missing,

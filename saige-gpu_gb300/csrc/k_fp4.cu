@@ -964,7 +964,8 @@ cudaError_t fp4_product(const void* Gmm, const void* Gsm, const float* Pf, int64
 //
 // with D_m fixed to integers (2 D_m <= 2^24).  The rows of B are samples: element m of row j is D_m g_jm, one of
 // 0, D_m, 2 D_m, in base-13 digits; the sums are exact, and so is the subtraction of a_i and a_j, which cancels
-// most of them: only D's rounding (2^-25 of its largest value) and the entry's own rounding to FP32 remain.
+// most of them: only D's rounding (2^-25 of its largest value) and the entry's two to FP32 (its sum, and the sum's
+// product with the scale) remain.
 // Against split-BF16's four products (off-diagonal error 4e-8 of entries of RMS 2.6e-3 at 100k x 150k, and row
 // sums off by n times its bias) this takes seven FP4 products, 1.2 BF16 ones' tensor time.
 namespace {

@@ -121,7 +121,7 @@ cudaError_t tc_wait_selftest(double budget_ms, int* waited_out, cudaStream_t s);
 // Shape options of the tcgen05 GEMMs (process-wide), in the order of sg_tc_option (saigegpu.h):
 // SYRK on CTA pairs, split-BF16 GRM.V on CTA pairs, drain length (bytes of K per row per TMEM
 // accumulator chunk), SYRK raster group (row tiles), split-BF16 GRM.V K slice bytes (0 = by width).
-// Then the subset-exact genotype GEMMs on CTA pairs (0 never, 1 always, 2 above 160 columns) and
+// Then the subset-exact genotype GEMMs on CTA pairs (0 never, 1 always, 2 except where the two-bit form serves) and
 // their K slice bytes (0 = by width).
 enum { kTcSyrkPair = 0, kTcGrmvPair = 1, kTcDrainBytes = 2, kTcSyrkGroup = 3, kTcGrmvSlice = 4, kTcSubsetPair = 5,
        kTcSubsetSlice = 6, kTcOptions = 7 };
@@ -301,7 +301,7 @@ cudaError_t fp4_product(const void* Gmm, const void* Gsm, const float* Pf, int64
                         int64_t m, const int32_t* cols, int64_t ncols, int ct, const ColState* st,
                         const SubsetSlot* slots, const double* winv, int max_w, const Fp4Scratch& w, float* Yf,
                         cudaStream_t s, int* launches);
-// The GRM from packed genotypes on the same pipe: K = Z Z' / M in exact integers, rounded once to FP32
+// The GRM from packed genotypes on the same pipe: K = Z Z' / M in exact integers, rounded to FP32 and scaled there
 struct Fp4SyrkPlan {
   bool ok = false;      // false: 1/sd^2 spans or spreads more than asked for, or too many markers
   int exponent = 0;     // 1/sd^2 is held as integers of 2^-exponent

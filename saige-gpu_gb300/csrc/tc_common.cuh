@@ -125,8 +125,7 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
-// One lane of a converged warp, by elect.sync: the compiler then keeps the operands of what that lane issues
-// (tcgen05.mma, TMA, commits) in uniform registers.  Behind a test of the lane number the same MMA loop took 45 clocks an
+// One lane of a converged warp, by elect.sync.  Behind a test of the lane number the same MMA loop took 45 clocks an
 // instruction, behind this 17 (128 x 32 x 16 BF16, its operands' own rate).
 __device__ __forceinline__ bool elect_one() {
   uint32_t e;
