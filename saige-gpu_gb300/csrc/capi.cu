@@ -289,7 +289,8 @@ struct sg_ctx {
   double* d_gk_p2d = nullptr;
   float *d_gk_dp = nullptr, *d_gk_p2 = nullptr;
   bool gk_refused = false;
-  double digit_spread = 0.0;  // of the GRM markers' 1/sd^2 (see fp32_form)
+  // of the GRM markers' 1/sd^2 (= d'): max d' times the mean (see fp32_form) and the RMS (see sg_grm_build) of sd^2
+  double digit_spread = 0.0, weight_spread = 0.0;
   bool k_exact = false;     // K holds the FP32-class GRM (not the single-product BF16 one)
   // synthetic bed image
   uint8_t* d_synth = nullptr;
@@ -797,14 +798,17 @@ static int setgeno_core(sg_ctx* c, const uint8_t* raw, int64_t raw_pitch, int64_
       c->vr_index.push_back((int32_t)i);
     }
   }
-  double wmax = 0.0, inv_sum = 0.0;
-  for (const float x : c->invstd)
-    if (x > 0.0f) {
-      const double w = (double)x * (double)x;
-      wmax = std::max(wmax, w);
-      inv_sum += 1.0 / w;
-    }
-  c->digit_spread = wmax * inv_sum / (double)std::max<size_t>(c->invstd.size(), 1);
+  float smax = 0.0f;
+  double var = 0.0, var2 = 0.0;
+  for (size_t i = 0; i < c->freq.size(); ++i) {  // sd^2 = 2p(1 - p): no division for each of the markers
+    const double p = c->freq[i], v = 2.0 * p * (1.0 - p);
+    smax = std::max(smax, c->invstd[i]);
+    var += v;
+    var2 += v * v;
+  }
+  const double wmax = (double)smax * smax, markers = (double)std::max<size_t>(c->freq.size(), 1);
+  c->digit_spread = wmax * (var / markers);
+  c->weight_spread = wmax * std::sqrt(var2 / markers);
   c->fill_all.resize(m_bim);
   for (int64_t i = 0; i < m_bim; ++i) c->fill_all[i] = qc[i].fill;
   c->qc_min_maf = min_maf;
@@ -1197,7 +1201,8 @@ extern "C" int sg_grm_build(sg_ctx* c, int precision) {
   c->np = np;
   if (!c->d_K) SG_TRY(dev_alloc_t(c, &c->d_K, (size_t)(np * np)));
   const float scale = 1.0f / (float)c->m_qc;
-  if (precision != SG_GRM_BF16_TC && tc_available()) {
+  if (precision != SG_GRM_BF16_TC && tc_available() &&
+      c->weight_spread <= fp4_syrk_spread(c->m_qc, precision == SG_GRM_BF16X3_TC)) {
     // Exact integers on the FP4 pipe (k_fp4.cu) where their rounding of 1/sd^2, common to all markers, costs no more than
     // the other build's own: while 1/sd^2 spans at most a factor of 200 (MAF above ~0.0013) and its ``spread``, max D times
     // the RMS of 1/D, is bounded.  Off-diagonal entries are then off by 4.9e-8 spread / sqrt(M) RMS.  Split BF16: 16-bit
@@ -1207,8 +1212,7 @@ extern "C" int sg_grm_build(sg_ctx* c, int precision) {
     // M = 700 with one marker of MAF 0.0013, spread 136: off-diagonals 2e-8 against 25e-8, left to FP32).
     std::vector<double> weight, centre;
     grm_weights(c, precision, weight, centre);
-    const Fp4SyrkPlan plan =
-        fp4_syrk_plan(weight.data(), c->m_qc, np, 200.0, fp4_syrk_spread(c->m_qc, precision == SG_GRM_BF16X3_TC));
+    const Fp4SyrkPlan plan = fp4_syrk_plan(weight.data(), c->m_qc, np, 200.0);
     void* scratch = nullptr;
     const std::string err = c->err;
     if (plan.ok && dev_alloc(c, &scratch, (size_t)plan.bytes) == SG_OK) {

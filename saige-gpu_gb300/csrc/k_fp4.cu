@@ -1046,28 +1046,25 @@ __global__ void fp4_shift_kernel(const long long* __restrict__ sums, int64_t ld,
 
 }  // namespace
 
+// Bound on max D times the RMS of 1/D, to which the entries' RMS error is in proportion (where the line lies: sg_grm_build).
 double fp4_syrk_spread(int64_t m, bool split_bf16) {
   if (split_bf16) return 80.0;
   return std::max(0.6 * std::sqrt((double)m), m >= 128 ? 24.0 : 0.0);
 }
 
-// Bytes of a build's scratch (see fp4_syrk), and whether integers of 24 bits hold D: the markers of the smallest D keep an
-// error of 2^-25 ``range`` relative at most, and the entries' RMS error is in proportion to ``spread`` (max D times the RMS of
-// 1/D).
-Fp4SyrkPlan fp4_syrk_plan(const double* weight, int64_t m, int64_t np, double range, double spread) {
+// Bytes of a build's scratch (see fp4_syrk), and whether D's range lets integers of 24 bits hold it: the markers of the
+// smallest D then keep an error of 2^-25 ``range`` relative at most.
+Fp4SyrkPlan fp4_syrk_plan(const double* weight, int64_t m, int64_t np, double range) {
   Fp4SyrkPlan p;
-  double lo = 1e300, hi = 0.0, inv2 = 0.0;
+  double lo = 1e300, hi = 0.0;
   for (int64_t i = 0; i < m; ++i) {
     const double d = weight[i];
     if (d > 0.0) {
       lo = d < lo ? d : lo;
       hi = d > hi ? d : hi;
-      inv2 += 1.0 / (d * d);
     }
   }
-  if (m <= 0 || !(hi > 0.0) || !(hi < 1e30) || hi > range * lo || !(hi * std::sqrt(inv2 / (double)m) <= spread) ||
-      fp4_stages(m) > kSegStages)
-    return p;
+  if (m <= 0 || !(hi > 0.0) || !(hi < 1e30) || hi > range * lo || fp4_stages(m) > kSegStages) return p;
   int e = 0;
   frexp(hi, &e);  // hi < 2^e
   p.exponent = 23 - e;

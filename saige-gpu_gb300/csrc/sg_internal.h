@@ -303,14 +303,14 @@ cudaError_t fp4_product(const void* Gmm, const void* Gsm, const float* Pf, int64
                         cudaStream_t s, int* launches);
 // The GRM from packed genotypes on the same pipe: K = Z Z' / M in exact integers, rounded to FP32 and scaled there
 struct Fp4SyrkPlan {
-  bool ok = false;      // false: 1/sd^2 spans or spreads more than asked for, or too many markers
+  bool ok = false;      // false: 1/sd^2 spans more than the range asked for, or too many markers
   int exponent = 0;     // 1/sd^2 is held as integers of 2^-exponent
   int64_t bytes = 0;    // scratch
   int64_t off_a = 0, off_b = 0, off_shift_b = 0, off_sums = 0, off_shift = 0, off_words = 0, off_hilo = 0, off_tiles = 0;
   std::vector<int32_t> tiles;
 };
-Fp4SyrkPlan fp4_syrk_plan(const double* weight, int64_t m, int64_t np, double range, double spread);
-double fp4_syrk_spread(int64_t m, bool split_bf16);  // the spread a build over m markers allows
+Fp4SyrkPlan fp4_syrk_plan(const double* weight, int64_t m, int64_t np, double range);
+double fp4_syrk_spread(int64_t m, bool split_bf16);  // the spread of 1/sd^2 that a build over m markers allows
 cudaError_t fp4_syrk(const Fp4SyrkPlan& plan, void* scratch, const uint8_t* packed, int64_t pitch, const double* weight,
                      const double* centre, int64_t m, int64_t n, int64_t np, float* K, cudaStream_t s);
 constexpr int kProbeDotsMaxP = 16;
